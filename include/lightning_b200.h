@@ -4,7 +4,7 @@
  *
  * Conventions
  *  - Every pointer is a CUDA device pointer owned by the caller unless stated otherwise; the
- *    library never allocates or frees device memory (its only allocation is 256 bytes of pinned host
+ *    library never allocates or frees device memory (its only allocation is one word of pinned host
  *    memory per device for lab200_last_status).
  *  - `stream` is a cudaStream_t passed as void*; all work is enqueued on it and the calls return
  *    without synchronising (except lab200_read_status).
@@ -210,13 +210,12 @@ int lab200_la2_dkdv(const void* q, const void* k, const void* v, const float* sl
 int lab200_read_status(const void* workspace, void* stream);
 
 /*
- * Status without a host synchronisation. After the last launch of every attention call that takes a workspace the
- * library enqueues a 4-byte copy of the call's status word into a ring (64 slots per device) of pinned host memory,
- * which it allocates with cudaHostAlloc on the first such call on a device (make that call outside stream capture).
- * lab200_last_status() looks through the ring of the current device and returns - and clears - the first non-zero word
- * (a LAB200_ERR_WAIT_* code: a bounded wait of an EARLIER call ran out and that call's outputs are invalid), or 0.
- * It never blocks; the report is at least one call late (the copy runs behind the kernels) and a word that is not
- * collected within 64 later calls is overwritten. The Python operators call it before every launch and raise.
+ * Status without a host synchronisation. A kernel whose bounded wait runs out writes its code into the workspace's status
+ * word and into one word of pinned host memory per device, which the library allocates with cudaHostAlloc on the first
+ * attention call on that device (make that call outside stream capture). lab200_last_status() returns - and clears - the
+ * current device's word: a LAB200_ERR_WAIT_* code if a bounded wait of an EARLIER call ran out (that call's outputs are
+ * invalid), or 0. It never blocks, so the report is at least one call late; of several reports the last one is kept.
+ * The Python operators call it before every launch and raise.
  * No counterpart in the reference (its kernels have no waits that can run out).
  */
 int lab200_last_status(void);
@@ -228,8 +227,7 @@ int lab200_static_status(void* stream);
 
 /* Test hook for the error path: one tiny kernel waits - with the bounded wait of the block kernels and a budget of
  * `budget_cycles` SM clocks (at most 1e8) - on a barrier nothing arrives on, so the wait runs out and the kernel writes
- * LAB200_ERR_WAIT_INPUT into the workspace's status word and returns; the call then posts the word like every attention
- * call does. No copy, tensor memory or MMA is in flight in that kernel. No counterpart in the reference. */
+ * LAB200_ERR_WAIT_INPUT into the status words, like the block kernels do, and returns. No copy, tensor memory or MMA is in flight in that kernel. No counterpart in the reference. */
 int lab200_debug_wait_expiry(void* workspace, size_t workspace_bytes, long long budget_cycles, void* stream);
 
 /* y = x * rsqrt(mean(x^2, last dim) + eps), rstd saved per row: _SrmsNorm.forward /

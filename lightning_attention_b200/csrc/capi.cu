@@ -212,6 +212,54 @@ int launch_la(int mode, int dtype, const Tiling& t, const CUtensorMap& tA, const
                               : launch_tiled<1, 0>(t.nks, t.nvs, tA, tB, tC, p, grid, smem, st);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Device status. A bounded wait that runs out is reported by the kernel itself, into the status word of the call's
+// workspace and into one word of pinned, device-mapped host memory per device (allocated on the first attention call on
+// that device), which lab200_last_status() reads and clears without synchronising.
+// ---------------------------------------------------------------------------------------------
+constexpr int MAX_DEVICES = 64;
+struct HostStatus {
+  int* word = nullptr;
+  bool tried = false;
+};
+HostStatus g_host_status[MAX_DEVICES];
+std::mutex g_status_mutex;
+
+// The current device's word, or nullptr (no device, or no pinned memory to be had: failures then only reach the workspace).
+int* host_status_word(bool allocate) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return nullptr;
+  std::lock_guard<std::mutex> lock(g_status_mutex);
+  HostStatus& hs = g_host_status[dev];
+  if (!hs.word && !hs.tried && allocate) {
+    hs.tried = true;
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped) == cudaSuccess && p) {
+      hs.word = static_cast<int*>(p);
+      *hs.word = 0;
+    } else {
+      cudaGetLastError();
+    }
+  }
+  return hs.word;
+}
+
+// Status destination of one call, handed to its launches in turn: the first block kernel clears the workspace word.
+struct CallStatus {
+  LaStatus st;
+  CallStatus(void* workspace, int* host) : st{static_cast<int*>(workspace), host, 1} {
+    // The tensor-map encoder is a driver call and needs the device's context to be current on this thread; on a thread that
+    // has made no runtime call yet (an autograd thread) only cudaSetDevice makes it so.
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaSetDevice(dev);
+  }
+  LaStatus next() {
+    const LaStatus r = st;
+    st.reset = 0;
+    return r;
+  }
+};
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 int la_validate(const void* a, const void* bm, const void* c, const void* out, const float* state_in,
@@ -235,7 +283,7 @@ int chunk_count(int bh, int n, int dk, int dv, int chunks) {
 int la_generic_impl(const void* a, const void* bm, const void* c, const float* slopes, void* out,
                     const float* state_in, float* state_out, void* workspace, size_t workspace_bytes, int bh, int h,
                     int n, int dk, int dv, int reverse, int state_only, int chunks, int dtype, cudaStream_t st,
-                    int resume = 0) {
+                    CallStatus& status, int resume = 0) {
   const bool prefix_only = (resume & PREFIX_ONLY) != 0;
   int rc = la_validate(a, bm, c, out, state_in, state_out, workspace, bh, h, n, dk, dv, prefix_only ? 2 : state_only, dtype);
   if (rc != LAB200_OK) return rc;
@@ -264,7 +312,6 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
   LaParams p;
   p.out = out;
   p.slopes = slopes;
-  p.status = static_cast<int*>(workspace);
   p.n = n; p.h = h; p.dk = dk; p.dv = dv;
   p.nblocks = nblocks;
   p.blocks_per_chunk = bpc;
@@ -281,6 +328,7 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
     p.state_slots = 1;
     p.state_in = state_in;
     p.state_out = state_out;
+    p.status = status.next();
     return launch_la(state_only ? 1 : 0, dtype, t, tA, tB, tC, tO, p, 1, bh, st);
   }
 
@@ -310,6 +358,7 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
     p.chunk0 = 0;
     p.state_in = states;
     p.state_out = nullptr;
+    p.status = status.next();
     return launch_la(0, dtype, t, tA, tB, tC, tO, p, nchunks, bh, st);
   }
   const bool need_total = (state_out != nullptr);
@@ -326,6 +375,7 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
     ts.nvs = 1;
     ts.nslices = (dv + 63) / 64;
   }
+  p.status = status.next();
   if ((rc = launch_la(1, dtype, ts, tB, tB, tC, tC, p, nchunks - skip_last, bh, st)) != LAB200_OK) return rc;
 
   const int elems = dv * dk;
@@ -341,6 +391,7 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
   p.chunk0 = 0;
   p.state_in = states;
   p.state_out = nullptr;
+  p.status = status.next();
   return launch_la(0, dtype, t, tA, tB, tC, tO, p, nchunks, bh, st);
 }
 
@@ -377,8 +428,8 @@ bool dkdv_shape_ok(int d, int e) { return d <= 128 && e <= 128 && (d % 16) == 0 
 // the reverse-time state entering every chunk, [bh][nchunks][d][e] fp32. Returns LAB200_ERR_SHAPE if the shape is not
 // covered, in which case the caller falls back to two generic launches.
 int la_dkdv_impl(const void* q, const void* k, const void* v, const void* dout, const float* slopes, void* dk, void* dv,
-                 void* workspace, const float* states, int nchunks, int bpc, int bh, int h, int n, int d, int e, int dtype,
-                 cudaStream_t st) {
+                 const float* states, int nchunks, int bpc, int bh, int h, int n, int d, int e, int dtype,
+                 cudaStream_t st, CallStatus& status) {
   const int layout = (dtype & LAB200_LAYOUT_BNHD) ? 1 : 0;
   dtype &= 0xff;
   if (!dkdv_shape_ok(d, e)) return LAB200_ERR_SHAPE;
@@ -397,7 +448,7 @@ int la_dkdv_impl(const void* q, const void* k, const void* v, const void* dout, 
   p.slopes = slopes;
   p.state_in = states;
   p.state_out = nullptr;
-  p.status = static_cast<int*>(workspace);
+  p.status = status.next();
   p.n = n; p.h = h; p.d = d; p.e = e;
   p.nblocks = (n + LA_BLOCK - 1) / LA_BLOCK;
   p.blocks_per_chunk = states ? bpc : p.nblocks;
@@ -424,7 +475,7 @@ int la_dkdv_impl(const void* q, const void* k, const void* v, const void* dout, 
 // launch over all chunks. state_in: (bh, d, e) fp32 state entering the sequence from its far end, or nullptr.
 int la_dkdv_full(const void* q, const void* k, const void* v, const void* dout, const float* slopes, void* dk, void* dv,
                  const float* state_in, void* workspace, size_t workspace_bytes, int bh, int h, int n, int d, int e,
-                 int chunks, int resume, int dtype, cudaStream_t st) {
+                 int chunks, int resume, int dtype, cudaStream_t st, CallStatus& status) {
   if (!dkdv_shape_ok(d, e)) return LAB200_ERR_SHAPE;
   const int nblocks = (n + LA_BLOCK - 1) / LA_BLOCK;
   const int nchunks = chunk_count(bh, n, e, d, chunks);
@@ -432,12 +483,12 @@ int la_dkdv_full(const void* q, const void* k, const void* v, const void* dout, 
   if (nchunks > 1) {
     // chunk states of the product (v, do, q): sum lambda^t q_t^T do_t laid out (d, e), exactly the kernel's dKV
     int rc = la_generic_impl(nullptr, dout, q, slopes, nullptr, state_in, nullptr, workspace, workspace_bytes, bh, h, n, e, d,
-                             1, 0, chunks, dtype, st, PREFIX_ONLY | (resume ? RESUME : 0));
+                             1, 0, chunks, dtype, st, status, PREFIX_ONLY | (resume ? RESUME : 0));
     if (rc != LAB200_OK) return rc;
     const float* states = reinterpret_cast<const float*>(static_cast<const uint8_t*>(workspace) + WS_HEADER);
-    return la_dkdv_impl(q, k, v, dout, slopes, dk, dv, workspace, states, nchunks, bpc, bh, h, n, d, e, dtype, st);
+    return la_dkdv_impl(q, k, v, dout, slopes, dk, dv, states, nchunks, bpc, bh, h, n, d, e, dtype, st, status);
   }
-  return la_dkdv_impl(q, k, v, dout, slopes, dk, dv, workspace, state_in, 1, nblocks, bh, h, n, d, e, dtype, st);
+  return la_dkdv_impl(q, k, v, dout, slopes, dk, dv, state_in, 1, nblocks, bh, h, n, d, e, dtype, st, status);
 }
 
 // A reverse-time sweep starts in the last block; the state arriving there is taken to sit at the end of a full tile.
@@ -465,10 +516,7 @@ int la_validate(const void* a, const void* bm, const void* c, const void* out, c
   return LAB200_OK;
 }
 
-int reset_status(void* workspace, size_t workspace_bytes, cudaStream_t st) {
-  if (!workspace || workspace_bytes < WS_HEADER) return LAB200_ERR_WORKSPACE;
-  return cudaMemsetAsync(workspace, 0, 16, st) == cudaSuccess ? LAB200_OK : LAB200_ERR_CUDA;
-}
+bool workspace_ok(const void* workspace, size_t workspace_bytes) { return workspace && workspace_bytes >= WS_HEADER; }
 
 // ---------------------------------------------------------------------------------------------
 // SRMSNorm launch selection
@@ -626,7 +674,6 @@ int srms_entry(bool fwd, const void* x, const void* dy, void* out, float* rstd, 
 // ---------------------------------------------------------------------------------------------
 static __device__ __align__(256) unsigned char g_static_scratch[LAB200_STATIC_SCRATCH_BYTES];
 
-constexpr int MAX_DEVICES = 64;
 void* g_static_scratch_addr[MAX_DEVICES] = {};
 std::mutex g_static_scratch_mutex;
 
@@ -651,50 +698,11 @@ int static_scratch_address(void** out) {
   return LAB200_OK;
 }
 
-// ---------------------------------------------------------------------------------------------
-// Device status without a host synchronisation: after the last launch of an attention call the library copies the
-// call's status word into a slot of a small ring of pinned host memory (one ring per device, allocated on the first
-// attention call on that device). lab200_last_status() scans the ring: a non-zero word means a bounded wait of an
-// EARLIER call ran out. The copy is ordered behind the call's kernels, so the report is one or more calls late.
-// ---------------------------------------------------------------------------------------------
-constexpr int STATUS_RING = 64;
-struct StatusRing {
-  int* slots = nullptr;
-  unsigned next = 0;
-  bool tried = false;
-};
-StatusRing g_status_ring[MAX_DEVICES];
-std::mutex g_status_mutex;
-
-void post_status(const void* workspace, cudaStream_t st) {
-  int dev = -1;
-  if (!workspace || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return;
-  std::lock_guard<std::mutex> lock(g_status_mutex);
-  StatusRing& ring = g_status_ring[dev];
-  if (!ring.slots && !ring.tried) {
-    ring.tried = true;
-    void* p = nullptr;
-    if (cudaHostAlloc(&p, STATUS_RING * sizeof(int), cudaHostAllocDefault) == cudaSuccess && p) {
-      ring.slots = static_cast<int*>(p);
-      for (int i = 0; i < STATUS_RING; ++i) ring.slots[i] = 0;
-    } else {
-      cudaGetLastError();
-    }
-  }
-  if (!ring.slots) return;
-  int* slot = ring.slots + (ring.next++ % STATUS_RING);
-  if (cudaMemcpyAsync(slot, workspace, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) cudaGetLastError();
-}
-
-int finish_call(int rc, const void* workspace, cudaStream_t st) {
-  if (rc == LAB200_OK) post_status(workspace, st);
-  return rc;
-}
-
 // One CTA that waits, with the same bounded wait the block kernels use, on an mbarrier that nothing ever arrives on, and
 // reports the expiry through the status word: exercises the error path (wait budget -> status word -> host) with no
 // asynchronous copy, tensor-memory allocation or MMA in flight.
-__global__ void la_wait_expiry_kernel(int* status, long long budget) {
+__global__ void la_wait_expiry_kernel(LaStatus status, long long budget) {
+  la_status_begin(status);
   __shared__ __align__(8) unsigned long long bar_storage;
   __shared__ int abort_flag;
   const uint32_t bar = smem_u32(&bar_storage);
@@ -706,7 +714,7 @@ __global__ void la_wait_expiry_kernel(int* status, long long budget) {
   __syncthreads();
   const bool ok = lap_wait(bar, 0, &abort_flag, budget);
   __syncthreads();
-  if (threadIdx.x == 0 && !ok) atomicExch(status, LA_ERR_WAIT_INPUT);
+  if (threadIdx.x == 0 && !ok) la_status_report(status, LA_ERR_WAIT_INPUT);
 }
 
 }  // namespace
@@ -758,9 +766,10 @@ int lab200_la_generic(const void* a, const void* bm, const void* c, const float*
   int rc = la_validate(a, bm, c, out, state_in, state_out, workspace, bh, h, n, dk, dv, state_only, dtype);
   if (rc != LAB200_OK) return rc;
   if (!reverse_chain_ok(reverse, state_in, n)) return LAB200_ERR_SHAPE;
-  if ((rc = reset_status(workspace, workspace_bytes, st)) != LAB200_OK) return rc;
-  return finish_call(la_generic_impl(a, bm, c, slopes, out, state_in, state_out, workspace, workspace_bytes, bh, h, n, dk, dv,
-                         reverse, state_only, chunks, dtype, st), workspace, st);
+  if (!workspace_ok(workspace, workspace_bytes)) return LAB200_ERR_WORKSPACE;
+  CallStatus status(workspace, host_status_word(true));
+  return la_generic_impl(a, bm, c, slopes, out, state_in, state_out, workspace, workspace_bytes, bh, h, n, dk, dv,
+                         reverse, state_only, chunks, dtype, st, status);
 }
 
 int lab200_la_generic_resume(const void* a, const void* bm, const void* c, const float* slopes, void* out,
@@ -770,9 +779,10 @@ int lab200_la_generic_resume(const void* a, const void* bm, const void* c, const
   int rc = la_validate(a, bm, c, out, state_in, nullptr, workspace, bh, h, n, dk, dv, 0, dtype);
   if (rc != LAB200_OK) return rc;
   if (!reverse_chain_ok(reverse, state_in, n)) return LAB200_ERR_SHAPE;
-  if ((rc = reset_status(workspace, workspace_bytes, st)) != LAB200_OK) return rc;
-  return finish_call(la_generic_impl(a, bm, c, slopes, out, state_in, nullptr, workspace, workspace_bytes, bh, h, n, dk, dv, reverse, 0,
-                         chunks, dtype, st, RESUME), workspace, st);
+  if (!workspace_ok(workspace, workspace_bytes)) return LAB200_ERR_WORKSPACE;
+  CallStatus status(workspace, host_status_word(true));
+  return la_generic_impl(a, bm, c, slopes, out, state_in, nullptr, workspace, workspace_bytes, bh, h, n, dk, dv, reverse, 0,
+                         chunks, dtype, st, status, RESUME);
 }
 
 int lab200_la_generic_resume_swapped(const void* a, const void* bm, const void* c, const float* slopes, void* out,
@@ -783,9 +793,10 @@ int lab200_la_generic_resume_swapped(const void* a, const void* bm, const void* 
   int rc = la_validate(a, bm, c, out, state_in, nullptr, workspace, bh, h, n, dk, dv, 0, dtype);
   if (rc != LAB200_OK) return rc;
   if (!reverse_chain_ok(reverse, state_in, n)) return LAB200_ERR_SHAPE;
-  if ((rc = reset_status(workspace, workspace_bytes, st)) != LAB200_OK) return rc;
-  return finish_call(la_generic_impl(a, bm, c, slopes, out, state_in, nullptr, workspace, workspace_bytes, bh, h, n, dk, dv, reverse, 0,
-                         chunks, dtype, st, RESUME | RESUME_SWAPPED | (rebase ? 0 : RESUME_NO_REBASE)), workspace, st);
+  if (!workspace_ok(workspace, workspace_bytes)) return LAB200_ERR_WORKSPACE;
+  CallStatus status(workspace, host_status_word(true));
+  return la_generic_impl(a, bm, c, slopes, out, state_in, nullptr, workspace, workspace_bytes, bh, h, n, dk, dv, reverse, 0,
+                         chunks, dtype, st, status, RESUME | RESUME_SWAPPED | (rebase ? 0 : RESUME_NO_REBASE));
 }
 
 int lab200_la_combine_states(const float* gathered, const float* slopes, float* out, float* out_t, int ranks, int rank,
@@ -825,9 +836,10 @@ int lab200_la2_fwd(const void* q, const void* k, const void* v, const float* slo
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc = la_validate(q, k, v, o, nullptr, nullptr, workspace, b * h, h, n, d, e, 0, dtype);
   if (rc != LAB200_OK) return rc;
-  if ((rc = reset_status(workspace, workspace_bytes, st)) != LAB200_OK) return rc;
-  return finish_call(la_generic_impl(q, k, v, slopes, o, nullptr, nullptr, workspace, workspace_bytes, b * h, h, n, d, e, 0, 0,
-                         chunks, dtype, st), workspace, st);
+  if (!workspace_ok(workspace, workspace_bytes)) return LAB200_ERR_WORKSPACE;
+  CallStatus status(workspace, host_status_word(true));
+  return la_generic_impl(q, k, v, slopes, o, nullptr, nullptr, workspace, workspace_bytes, b * h, h, n, d, e, 0, 0,
+                         chunks, dtype, st, status);
 }
 
 int lab200_la2_fwd_static(const void* q, const void* k, const void* v, const float* slopes, void* o, int b, int h,
@@ -844,12 +856,12 @@ int lab200_la2_fwd_static(const void* q, const void* k, const void* v, const flo
   if ((rc = static_scratch_address(&scratch)) != LAB200_OK) return rc;
   // the array keeps whatever the previous call left: the status word must start at zero; the chunk states
   // need no clearing because the state kernel writes every slot that the scan reads
-  if ((rc = reset_status(scratch, LAB200_STATIC_SCRATCH_BYTES, st)) != LAB200_OK) return rc;
+  CallStatus status(scratch, nullptr);
   return la_generic_impl(q, k, v, slopes, o, nullptr, nullptr, scratch, LAB200_STATIC_SCRATCH_BYTES, b * h, h, n, d, e,
-                         0, 0, chunks, dtype, st);
+                         0, 0, chunks, dtype, st, status);
 }
 
-static int la2_bwd_body(const void* q, const void* k, const void* v, const float* slopes, const void* dout, void* dq,
+int lab200_la2_bwd(const void* q, const void* k, const void* v, const float* slopes, const void* dout, void* dq,
                    void* dk, void* dv, void* workspace, size_t workspace_bytes, int b, int h, int n, int d, int e,
                    int chunks, int dtype, void* stream) {
   if (b < 1 || h < 1 || b > 65535 / h) return LAB200_ERR_SHAPE;
@@ -859,33 +871,26 @@ static int la2_bwd_body(const void* q, const void* k, const void* v, const float
   if (rc == LAB200_OK) rc = la_validate(k, q, dout, dv, nullptr, nullptr, workspace, bh, h, n, d, e, 0, dtype);
   if (rc == LAB200_OK && (!q || !dk || !aligned16(q) || !aligned16(dk))) rc = q && dk ? LAB200_ERR_ALIGN : LAB200_ERR_SHAPE;
   if (rc != LAB200_OK) return rc;
-  if ((rc = reset_status(workspace, workspace_bytes, st)) != LAB200_OK) return rc;
+  if (!workspace_ok(workspace, workspace_bytes)) return LAB200_ERR_WORKSPACE;
+  CallStatus status(workspace, host_status_word(true));
   // dq_t = sum_{j<=t} lambda^(t-j) (do_t . v_j) k_j
   rc = la_generic_impl(dout, v, k, slopes, dq, nullptr, nullptr, workspace, workspace_bytes, bh, h, n, e, d, 0, 0,
-                       chunks, dtype, st);
+                       chunks, dtype, st, status);
   if (rc != LAB200_OK) return rc;
   // dk_t = sum_{j>=t} lambda^(j-t) (v_t . do_j) q_j  and  dv_t = sum_{j>=t} lambda^(j-t) (k_t . q_j) do_j:
   // one fused reverse sweep (d, e <= 128), else two launches of the generic kernel
   if (use_fused_dkdv() && dkdv_shape_ok(d, e)) {
-    rc = la_dkdv_full(q, k, v, dout, slopes, dk, dv, nullptr, workspace, workspace_bytes, bh, h, n, d, e, chunks, 0, dtype, st);
+    rc = la_dkdv_full(q, k, v, dout, slopes, dk, dv, nullptr, workspace, workspace_bytes, bh, h, n, d, e, chunks, 0, dtype, st, status);
     if (rc != LAB200_ERR_SHAPE) return rc;
   }
   rc = la_generic_impl(v, dout, q, slopes, dk, nullptr, nullptr, workspace, workspace_bytes, bh, h, n, e, d, 1, 0,
-                       chunks, dtype, st);
+                       chunks, dtype, st, status);
   if (rc != LAB200_OK) return rc;
   // In chunk mode the dk launch leaves the reverse-time state entering every chunk, sum lambda^t q_t^T do_t as (d, e), in
   // the workspace; dv needs the same states as (e, d). With d == e they are transposed in place instead of recomputed.
   const int resume = (d == e && chunk_count(bh, n, e, d, chunks) > 1) ? (RESUME | RESUME_SWAPPED | RESUME_NO_REBASE) : 0;
   return la_generic_impl(k, q, dout, slopes, dv, nullptr, nullptr, workspace, workspace_bytes, bh, h, n, d, e, 1, 0,
-                         chunks, dtype, st, resume);
-}
-
-int lab200_la2_bwd(const void* q, const void* k, const void* v, const float* slopes, const void* dout, void* dq,
-                   void* dk, void* dv, void* workspace, size_t workspace_bytes, int b, int h, int n, int d, int e,
-                   int chunks, int dtype, void* stream) {
-  return finish_call(la2_bwd_body(q, k, v, slopes, dout, dq, dk, dv, workspace, workspace_bytes, b, h, n, d, e, chunks, dtype,
-                                  stream),
-                     workspace, static_cast<cudaStream_t>(stream));
+                         chunks, dtype, st, status, resume);
 }
 
 size_t lab200_la2_bwd_workspace_bytes(int b, int h, int n, int d, int e, int chunks) {
@@ -909,10 +914,10 @@ int lab200_la2_dkdv(const void* q, const void* k, const void* v, const float* sl
   if ((dtype & LAB200_LAYOUT_BNHD) && static_cast<long long>(b) * h * n >= (1LL << 31)) return LAB200_ERR_SHAPE;
   if (!reverse_chain_ok(1, state_in, n)) return LAB200_ERR_SHAPE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int rc = reset_status(workspace, workspace_bytes, st);
-  if (rc != LAB200_OK) return rc;
-  return finish_call(la_dkdv_full(q, k, v, dout, slopes, dk, dv, state_in, workspace, workspace_bytes, b * h, h, n, d, e, chunks,
-                      resume, dtype, st), workspace, st);
+  if (!workspace_ok(workspace, workspace_bytes)) return LAB200_ERR_WORKSPACE;
+  CallStatus status(workspace, host_status_word(true));
+  return la_dkdv_full(q, k, v, dout, slopes, dk, dv, state_in, workspace, workspace_bytes, b * h, h, n, d, e, chunks,
+                      resume, dtype, st, status);
 }
 
 int lab200_read_status(const void* workspace, void* stream) {
@@ -925,19 +930,11 @@ int lab200_read_status(const void* workspace, void* stream) {
 }
 
 int lab200_last_status(void) {
-  int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return 0;
-  std::lock_guard<std::mutex> lock(g_status_mutex);
-  StatusRing& ring = g_status_ring[dev];
-  if (!ring.slots) return 0;
-  for (int i = 0; i < STATUS_RING; ++i) {
-    const int v = *const_cast<volatile int*>(ring.slots + i);
-    if (v != 0) {
-      ring.slots[i] = 0;
-      return v;
-    }
-  }
-  return 0;
+  int* word = host_status_word(false);
+  if (!word) return 0;
+  const int v = *const_cast<volatile int*>(word);
+  if (v != 0) *const_cast<volatile int*>(word) = 0;
+  return v;
 }
 
 int lab200_static_status(void* stream) {
@@ -949,13 +946,11 @@ int lab200_static_status(void* stream) {
 int lab200_debug_wait_expiry(void* workspace, size_t workspace_bytes, long long budget_cycles, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (budget_cycles < 1 || budget_cycles > 100000000LL) return LAB200_ERR_SHAPE;  // at most ~50 ms of SM clocks
-  int rc = reset_status(workspace, workspace_bytes, st);
-  if (rc != LAB200_OK) return rc;
-  la_wait_expiry_kernel<<<1, 32, 0, st>>>(static_cast<int*>(workspace), budget_cycles);
+  if (!workspace_ok(workspace, workspace_bytes)) return LAB200_ERR_WORKSPACE;
+  CallStatus status(workspace, host_status_word(true));
+  la_wait_expiry_kernel<<<1, 32, 0, st>>>(status.next(), budget_cycles);
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (cudaGetLastError() != cudaSuccess) return LAB200_ERR_CUDA;
-  post_status(workspace, st);
-  return LAB200_OK;
+  return cudaGetLastError() == cudaSuccess ? LAB200_OK : LAB200_ERR_CUDA;
 }
 
 int lab200_srmsnorm_fwd(const void* x, void* y, float* rstd, long long M, int N, float eps, int dtype, void* stream) {

@@ -42,7 +42,7 @@ struct LaDkdvParams {
   const float* slopes;     // [h] decay rates or nullptr
   const float* state_in;   // [bh][state_slots][d][e] fp32 reverse-time state entering the (chunk of the) sequence, or nullptr
   float* state_out;        // same indexing, or nullptr
-  int* status;
+  LaStatus status;
   int n, h, d, e;
   int nblocks, blocks_per_chunk, chunk0, state_slots;
   int layout;
@@ -116,6 +116,7 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const float s = p.slopes ? p.slopes[bh % p.h] : 0.f;
   const float s2 = -s * 1.4426950408889634f;
 
+  la_status_begin(p.status);
   if (tid == 0) {
     for (int i = 0; i < LD2_NUM_BARS; ++i) {
       uint32_t count = 1u;
@@ -613,7 +614,7 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   tc_fence_before_sync();
   __syncthreads();
-  if (tid == 0 && *abort_flag) atomicExch(p.status, *fail_code ? *fail_code : LA_ERR_WAIT_MMA2);
+  if (tid == 0 && *abort_flag) la_status_report(p.status, *fail_code ? *fail_code : LA_ERR_WAIT_MMA2);
   if (warp == 0) {
     __syncwarp();
     tmem_dealloc(tmem, 512);

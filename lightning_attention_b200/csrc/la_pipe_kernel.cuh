@@ -113,6 +113,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const float s = p.slopes ? p.slopes[bh % p.h] : 0.f;
   const float s2 = -s * 1.4426950408889634f;
 
+  la_status_begin(p.status);
   if (tid == 0) {
     for (int i = 0; i < LAP_NUM_BARS; ++i) {
       const uint32_t count = (i == LAP_P_READY) ? LAP_MASK_THREADS
@@ -527,7 +528,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   tc_fence_before_sync();
   __syncthreads();
-  if (tid == 0 && *abort_flag) atomicExch(p.status, *fail_code ? *fail_code : LA_ERR_WAIT_MMA2);
+  if (tid == 0 && *abort_flag) la_status_report(p.status, *fail_code ? *fail_code : LA_ERR_WAIT_MMA2);
   if (warp == 0) {
     __syncwarp();
     tmem_dealloc(tmem, 512);
