@@ -378,12 +378,11 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
   p.status = status.next();
   if ((rc = launch_la(1, dtype, ts, tB, tB, tC, tC, p, nchunks - skip_last, bh, st)) != LAB200_OK) return rc;
 
-  const int elems = dv * dk;
-  const long long total = static_cast<long long>(bh) * elems;
-  const int threads = 256;
-  const unsigned blocks = static_cast<unsigned>((total + threads - 1) / threads);
-  la_scan_kernel<<<blocks, threads, 0, st>>>(states, state_in, state_out, slopes, h, nchunks, elems, nblocks, bpc, n,
-                                             p.reverse, skip_last, total);
+  const int elems4 = dv * dk / 4;
+  const long long total = static_cast<long long>(bh) * elems4;
+  la_scan_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(
+      reinterpret_cast<float4*>(states), reinterpret_cast<const float4*>(state_in), reinterpret_cast<float4*>(state_out), slopes, h,
+      nchunks, elems4, nblocks, bpc, n, p.reverse, skip_last, total);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (cudaGetLastError() != cudaSuccess) return LAB200_ERR_CUDA;
   if (state_only || prefix_only) return LAB200_OK;
