@@ -261,6 +261,7 @@ struct CallStatus {
 };
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
 
 int la_validate(const void* a, const void* bm, const void* c, const void* out, const float* state_in,
                 const float* state_out, const void* workspace, int bh, int h, int n, int dk, int dv, int state_only,
@@ -517,11 +518,30 @@ int la_validate(const void* a, const void* bm, const void* c, const void* out, c
 
 bool workspace_ok(const void* workspace, size_t workspace_bytes) { return workspace && workspace_bytes >= WS_HEADER; }
 
+template <int FMT, int W, int LPR, int R>
+int launch_decode_one(const uint16_t* q, const uint16_t* k, const uint16_t* v, const float* slopes, float* state, uint16_t* o,
+                      int bh, int h, int dk, int dv, cudaStream_t st) {
+  constexpr int rows = LA_DECODE_THREADS / LPR * R;  // rows per CTA
+  la_decode_kernel<FMT, W, LPR, R><<<dim3((dv + rows - 1) / rows, bh), LA_DECODE_THREADS, 0, st>>>(q, k, v, slopes, state, o, h, dk, dv);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError() == cudaSuccess ? LAB200_OK : LAB200_ERR_CUDA;
+}
+
+template <int FMT>
+int launch_decode(const uint16_t* q, const uint16_t* k, const uint16_t* v, const float* slopes, float* state, uint16_t* o,
+                  int bh, int h, int dk, int dv, cudaStream_t st) {
+  // A row takes dk / 8 lanes: the smallest power of two that holds them is used, so that rows up to 256 wide are one access per
+  // lane (dk = 96 and 192 leave a quarter of the lanes idle, which a kernel bound by memory does not notice: 6.4 and 6.6 TB/s
+  // against 4.1 and 5.2 with 16-byte accesses over 32 lanes). A state that is only 16-byte aligned takes those.
+  if (!aligned32(state)) return launch_decode_one<FMT, 1, 32, 8>(q, k, v, slopes, state, o, bh, h, dk, dv, st);
+  if (dk <= 64) return launch_decode_one<FMT, 2, 8, LA_DECODE_R>(q, k, v, slopes, state, o, bh, h, dk, dv, st);
+  if (dk <= 128) return launch_decode_one<FMT, 2, 16, LA_DECODE_R>(q, k, v, slopes, state, o, bh, h, dk, dv, st);
+  return launch_decode_one<FMT, 2, 32, LA_DECODE_R>(q, k, v, slopes, state, o, bh, h, dk, dv, st);
+}
+
 // ---------------------------------------------------------------------------------------------
 // SRMSNorm launch selection
 // ---------------------------------------------------------------------------------------------
-bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
-
 // LIGHTNING_B200_SRMS_WIDE=0 keeps every SRMSNorm kernel on 128-bit accesses (A/B comparisons).
 bool use_wide_srms() {
   static const bool on = [] {
@@ -818,15 +838,12 @@ int lab200_la_decode_step(const void* q, const void* k, const void* v, const flo
   if (dtype != LAB200_BF16 && dtype != LAB200_F16) return LAB200_ERR_DTYPE;
   if (!aligned16(q) || !aligned16(k) || !aligned16(state)) return LAB200_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const dim3 grid((dv + 8 * LA_DECODE_ROWS - 1) / (8 * LA_DECODE_ROWS), bh);
   auto qq = static_cast<const uint16_t*>(q);
   auto kk = static_cast<const uint16_t*>(k);
   auto vv = static_cast<const uint16_t*>(v);
   auto oo = static_cast<uint16_t*>(o);
-  if (dtype == LAB200_BF16) la_decode_kernel<1><<<grid, 256, 0, st>>>(qq, kk, vv, slopes, state, oo, h, dk, dv);
-  else la_decode_kernel<0><<<grid, 256, 0, st>>>(qq, kk, vv, slopes, state, oo, h, dk, dv);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? LAB200_OK : LAB200_ERR_CUDA;
+  return dtype == LAB200_BF16 ? launch_decode<1>(qq, kk, vv, slopes, state, oo, bh, h, dk, dv, st)
+                              : launch_decode<0>(qq, kk, vv, slopes, state, oo, bh, h, dk, dv, st);
 }
 
 int lab200_la2_fwd(const void* q, const void* k, const void* v, const float* slopes, void* o, void* workspace,

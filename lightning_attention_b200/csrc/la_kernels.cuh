@@ -601,74 +601,105 @@ __global__ void la_transpose_square_kernel(float* __restrict__ m, int D) {
 
 // One decode step of the recurrence for every (batch, head) pair (inference; no counterpart in the reference):
 //   o = q (S + k^T v),   S <- lambda (S + k^T v),
-// S being the (dv, dk) fp32 state entering the token (what the block kernels hand out as state_out). A warp owns
-// LA_DECODE_ROWS state rows and keeps one 16-byte load per row in flight; 8 warps per CTA: grid
-// (ceil(dv / (8 LA_DECODE_ROWS)), bh), block 256. HBM-bound on the state: 8 bytes per element.
-constexpr int LA_DECODE_ROWS = 8;
+// S being the (dv, dk) fp32 state entering the token (what the block kernels hand out as state_out). HBM-bound on the state,
+// 8 bytes per element. Every state element is read once and written back once, so both go in 256-bit accesses marked
+// evict-first: 256 sequences x 32 heads x 128 x 128 take 156 us = 6.9 TB/s, 162 without the mark, 194 with 16-byte accesses.
+// CTAs are small and rows per warp few, because a CTA's loads, reduction and stores do not overlap each other: 256 threads with
+// the same rows per warp take 164 us, 64 x 64 states 111 against 80 us (16-byte accesses, 8 rows per warp, 256 threads: 157).
+constexpr int LA_DECODE_THREADS = 128;
+constexpr int LA_DECODE_R = 4;  // row accesses in flight per lane
+
+template <int W> struct LaStateVec { float f[4 * W]; };
+__device__ __forceinline__ void la_state_ld(LaStateVec<2>& v, const float* p) {
+  asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v.f[0]), "=f"(v.f[1]), "=f"(v.f[2]), "=f"(v.f[3]), "=f"(v.f[4]), "=f"(v.f[5]), "=f"(v.f[6]), "=f"(v.f[7])
+               : "l"(p));
+}
+__device__ __forceinline__ void la_state_st(float* p, const LaStateVec<2>& v) {
+  asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v.f[0]), "f"(v.f[1]),
+               "f"(v.f[2]), "f"(v.f[3]), "f"(v.f[4]), "f"(v.f[5]), "f"(v.f[6]), "f"(v.f[7]) : "memory");
+}
+__device__ __forceinline__ void la_state_ld(LaStateVec<1>& v, const float* p) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v.f[0] = t.x; v.f[1] = t.y; v.f[2] = t.z; v.f[3] = t.w;
+}
+__device__ __forceinline__ void la_state_st(float* p, const LaStateVec<1>& v) {
+  *reinterpret_cast<float4*>(p) = make_float4(v.f[0], v.f[1], v.f[2], v.f[3]);
+}
 
 template <int FMT>
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ uint16_t to_16bit(float x) {
+  if constexpr (FMT == 1) {
+    const __nv_bfloat16 b = __float2bfloat16_rn(x);
+    return *reinterpret_cast<const uint16_t*>(&b);
+  } else {
+    const __half hh = __float2half_rn(x);
+    return *reinterpret_cast<const uint16_t*>(&hh);
+  }
+}
+template <int FMT>
+__device__ __forceinline__ float from_16bit(uint16_t x) {
+  if constexpr (FMT == 1) return __uint_as_float(static_cast<uint32_t>(x) << 16);
+  else return __half2float(__ushort_as_half(x));
+}
+
+// Grid (ceil(dv / rows per CTA), bh). LPR lanes share a state row, each with 4 W neighbouring elements per access; a warp owns 32 / LPR * R rows, R accesses in flight.
+template <int FMT, int W, int LPR, int R>
+__global__ void __launch_bounds__(LA_DECODE_THREADS)
 la_decode_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k, const uint16_t* __restrict__ v,
                  const float* __restrict__ slopes, float* __restrict__ state, uint16_t* __restrict__ o, int h, int dk,
                  int dv) {
+  constexpr int EPL = 4 * W, RPW = 32 / LPR;
+  static_assert(R <= LPR, "lane j of a row's group writes the j-th result");
   const int bh = blockIdx.y;
-  const int row0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * LA_DECODE_ROWS;
-  const int lane = threadIdx.x & 31;
-  if (row0 >= dv) return;
-  const float lam = slopes ? __expf(-slopes[bh % h]) : 1.f;
-  auto to_f = [](uint32_t x) -> float {  // low 16 bits of x
-    if constexpr (FMT == 1) return __uint_as_float(x << 16);
-    else return __half2float(__ushort_as_half(static_cast<unsigned short>(x & 0xffffu)));
-  };
-  float ve[LA_DECODE_ROWS], acc[LA_DECODE_ROWS];
+  const int lane = threadIdx.x & 31, sub = lane % LPR;
+  const int row0 = (blockIdx.x * (LA_DECODE_THREADS / 32) + (threadIdx.x >> 5)) * (RPW * R) + lane / LPR;  // rows row0 + j RPW
+  float ve[R], acc[R];
 #pragma unroll
-  for (int j = 0; j < LA_DECODE_ROWS; ++j) {
-    ve[j] = (row0 + j < dv) ? to_f(v[static_cast<size_t>(bh) * dv + row0 + j]) : 0.f;
+  for (int j = 0; j < R; ++j) {
+    ve[j] = (row0 + j * RPW < dv) ? from_16bit<FMT>(v[static_cast<size_t>(bh) * dv + row0 + j * RPW]) : 0.f;
     acc[j] = 0.f;
   }
+  const float lam = slopes ? __expf(-slopes[bh % h]) : 1.f;
   const uint16_t* qp = q + static_cast<size_t>(bh) * dk;
   const uint16_t* kp = k + static_cast<size_t>(bh) * dk;
   float* sp = state + (static_cast<size_t>(bh) * dv + row0) * dk;
-  for (int c = lane * 4; c < dk; c += 128) {
-    float4 st[LA_DECODE_ROWS];
+  for (int c = sub * EPL; c < dk; c += LPR * EPL) {
+    LaStateVec<W> st[R];
 #pragma unroll
-    for (int j = 0; j < LA_DECODE_ROWS; ++j)
-      st[j] = (row0 + j < dv) ? *reinterpret_cast<const float4*>(sp + static_cast<size_t>(j) * dk + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const uint2 qq = *reinterpret_cast<const uint2*>(qp + c);
-    const uint2 kk = *reinterpret_cast<const uint2*>(kp + c);
-    const float k0 = to_f(kk.x & 0xffffu), k1 = to_f(kk.x >> 16), k2 = to_f(kk.y & 0xffffu), k3 = to_f(kk.y >> 16);
-    const float q0 = to_f(qq.x & 0xffffu), q1 = to_f(qq.x >> 16), q2 = to_f(qq.y & 0xffffu), q3 = to_f(qq.y >> 16);
+    for (int j = 0; j < R; ++j)
+      if (row0 + j * RPW < dv) la_state_ld(st[j], sp + static_cast<size_t>(j * RPW) * dk + c);
+    float kf[EPL], qf[EPL];
 #pragma unroll
-    for (int j = 0; j < LA_DECODE_ROWS; ++j) {
-      float4 nw;
-      nw.x = fmaf(k0, ve[j], st[j].x);
-      nw.y = fmaf(k1, ve[j], st[j].y);
-      nw.z = fmaf(k2, ve[j], st[j].z);
-      nw.w = fmaf(k3, ve[j], st[j].w);
-      acc[j] = fmaf(q0, nw.x, fmaf(q1, nw.y, fmaf(q2, nw.z, fmaf(q3, nw.w, acc[j]))));
-      if (row0 + j < dv)
-        *reinterpret_cast<float4*>(sp + static_cast<size_t>(j) * dk + c) = make_float4(lam * nw.x, lam * nw.y, lam * nw.z, lam * nw.w);
+    for (int i = 0; i < EPL; i += 4) {
+      const uint2 qq = *reinterpret_cast<const uint2*>(qp + c + i), kk = *reinterpret_cast<const uint2*>(kp + c + i);
+      kf[i] = from_16bit<FMT>(kk.x & 0xffffu); kf[i + 1] = from_16bit<FMT>(kk.x >> 16);
+      kf[i + 2] = from_16bit<FMT>(kk.y & 0xffffu); kf[i + 3] = from_16bit<FMT>(kk.y >> 16);
+      qf[i] = from_16bit<FMT>(qq.x & 0xffffu); qf[i + 1] = from_16bit<FMT>(qq.x >> 16);
+      qf[i + 2] = from_16bit<FMT>(qq.y & 0xffffu); qf[i + 3] = from_16bit<FMT>(qq.y >> 16);
+    }
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      if (row0 + j * RPW < dv) {
+#pragma unroll
+        for (int i = 0; i < EPL; ++i) {
+          const float nw = fmaf(kf[i], ve[j], st[j].f[i]);
+          acc[j] = fmaf(qf[i], nw, acc[j]);
+          st[j].f[i] = lam * nw;
+        }
+        la_state_st(sp + static_cast<size_t>(j * RPW) * dk + c, st[j]);
+      }
     }
   }
 #pragma unroll
-  for (int j = 0; j < LA_DECODE_ROWS; ++j) {
+  for (int j = 0; j < R; ++j) {
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], off);
+    for (int off = LPR / 2; off > 0; off >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], off);
   }
-  if (lane < LA_DECODE_ROWS && row0 + lane < dv) {
-    float mine = acc[0];
+  float mine = acc[0];
 #pragma unroll
-    for (int j = 1; j < LA_DECODE_ROWS; ++j) mine = (lane == j) ? acc[j] : mine;
-    uint16_t out;
-    if constexpr (FMT == 1) {
-      const __nv_bfloat16 bb = __float2bfloat16_rn(mine);
-      out = *reinterpret_cast<const uint16_t*>(&bb);
-    } else {
-      const __half hh = __float2half_rn(mine);
-      out = *reinterpret_cast<const uint16_t*>(&hh);
-    }
-    o[static_cast<size_t>(bh) * dv + row0 + lane] = out;
-  }
+  for (int j = 1; j < R; ++j) mine = (sub == j) ? acc[j] : mine;
+  if (sub < R && row0 + sub * RPW < dv) o[static_cast<size_t>(bh) * dv + row0 + sub * RPW] = to_16bit<FMT>(mine);
 }
 
 }  // namespace lab200

@@ -536,6 +536,27 @@ def test_decode_step_against_numpy_oracle(cuda_lib):
         la.lightning_attn_decode(q, k, v, s, st.transpose(2, 3))
 
 
+@pytest.mark.parametrize("d", [16, 64, 80, 128, 144, 256, 320])
+@pytest.mark.parametrize("e", [1, 17, 128])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_decode_step_at_the_edges_of_its_row_split(cuda_lib, d, e, offset):
+    """Row widths that fill and do not fill their lanes, rows left over, a state that is 16-byte but not 32-byte aligned."""
+    torch.manual_seed(24)
+    b, h = 2, 3
+    q, k = (torch.randn((b, h, d), device=DEV).bfloat16() for _ in range(2))
+    v = torch.randn((b, h, e), device=DEV).bfloat16()
+    buf = torch.full((b * h * e * d + 16,), 7.0, device=DEV)
+    st = buf[offset:offset + b * h * e * d].view(b, h, e, d)
+    st.copy_(torch.randn((b, h, e, d), device=DEV))
+    s = la._build_slope_tensor(h).to(DEV)
+    f = lambda t: t.float().cpu().numpy()
+    ro, rst = O.decode_step(f(q), f(k), f(v), f(s), f(st))
+    o = la.lightning_attn_decode(q, k, v, s, st)
+    assert O.rel_l2_err(f(o), ro) <= 2.0 ** -8  # one rounding to bf16 per element, at most half an ulp = 2^-9 relative
+    assert O.rel_l2_err(f(st), rst) <= 1e-6
+    assert (buf[:offset] == 7.0).all() and (buf[offset + b * h * e * d:] == 7.0).all()
+
+
 @pytest.mark.parametrize("b,h,n,d,e", [(4, 32, 512, 128, 128), (1, 4, 4096, 128, 128), (2, 3, 300, 64, 96), (1, 8, 2048, 128, 64),
                                        (2, 12, 384, 192, 192)])
 @pytest.mark.parametrize("decay", [True, False])
