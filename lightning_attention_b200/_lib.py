@@ -77,6 +77,28 @@ def lib():
     return _lib
 
 
+_host = None
+_HOST_ENTRIES = ("lab200_error_string", "lab200_last_status", "lab200_la_plan_chunks", "lab200_la_workspace_bytes", "lab200_la_generic",
+                 "lab200_la_generic_resume_swapped", "lab200_la_decode_step", "lab200_la2_fwd", "lab200_la2_bwd",
+                 "lab200_la2_bwd_workspace_bytes", "lab200_la2_dkdv", "lab200_srmsnorm_fwd", "lab200_srmsnorm_bwd",
+                 "lab200_srmsnorm_gate_fwd", "lab200_srmsnorm_gate_bwd")
+
+
+def host():
+    """The native call path (_host_ops.so), bound to the entry points of the loaded library."""
+    global _host
+    if _host is None:
+        L = lib()
+        try:
+            from . import _host_ops
+        except ImportError as ex:
+            raise ImportError(f"_host_ops.so is missing or does not load ({ex}): build it with "
+                              "`python -m lightning_attention_b200.build`") from ex
+        _host_ops.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in _HOST_ENTRIES})
+        _host = _host_ops
+    return _host
+
+
 EXPORTS = [
     "lab200_version", "lab200_launch_count", "lab200_la_debug_trace", "lab200_error_string", "lab200_la_plan_chunks", "lab200_la_workspace_bytes",
     "lab200_la_generic", "lab200_la_generic_resume", "lab200_la_generic_resume_swapped", "lab200_la_combine_states", "lab200_la_decode_step", "lab200_la2_fwd", "lab200_la2_fwd_static", "lab200_la2_bwd", "lab200_la2_bwd_workspace_bytes", "lab200_la2_dkdv", "lab200_read_status", "lab200_last_status", "lab200_static_status", "lab200_debug_wait_expiry",

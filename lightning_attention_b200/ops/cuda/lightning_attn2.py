@@ -5,6 +5,9 @@ Mirrors the operator layer of the reference: ``LightningAttention2`` / ``lightni
 ``lightning_attn2_no_decay`` (lightning_attn2_no_decay.py:367-471). Inputs are made contiguous,
 outputs are allocated here with torch, (q, k, v, s) are saved for backward, and ``s`` receives no
 gradient, exactly as there. All device work goes through the C ABI on the current CUDA stream.
+
+The public operators at the end try the native call path first (csrc/host_ops.cpp: the same checks, allocations, protocol and
+C-ABI calls without Python in between), which answers None to every call that is not of the common form.
 """
 import torch
 
@@ -342,6 +345,10 @@ def lightning_attn_prefill(q, k, v, s=None, kv_state=None):
     state entering the first token, i.e. what an earlier call returned. Returns (o, kv_state_out) where kv_state_out
     is the state entering token n: sum_{j<n} lambda^(n-j) k_j^T v_j (transposed) plus the decayed incoming state.
     Feeding it to the next prefill chunk or to `lightning_attn_decode` continues the sequence exactly."""
+    if not torch.compiler.is_compiling():
+        r = _lib.host().prefill(q, k, v, s, kv_state)
+        if r is not None:
+            return r
     _check_inputs(q, k, v)
     with torch.no_grad():
         o, st = la_generic(q.detach(), k.detach(), v.detach(), None if s is None else s.detach(), state_in=kv_state,
@@ -354,6 +361,10 @@ def lightning_attn_decode(q, k, v, s, kv_state):
 
     q, k: (b, h, d) or (b, h, 1, d); v: (b, h, e) or (b, h, 1, e); kv_state: (b, h, e, d) fp32 contiguous, from
     `lightning_attn_prefill` (or zeros for an empty prefix). Returns o shaped like v. No autograd."""
+    if not torch.compiler.is_compiling():
+        o = _lib.host().decode(q, k, v, s, kv_state)
+        if o is not None:
+            return o
     _lib.require_cuda(q, k, v, kv_state)
     squeeze = q.dim() == 4
     if squeeze:
@@ -377,8 +388,24 @@ def lightning_attn_decode(q, k, v, s, kv_state):
     return o.unsqueeze(2) if squeeze else o
 
 
-lightning_attn2 = LightningAttention2.apply
-lightning_attn2_no_decay = LightningAttention2NoDecay.apply
+def lightning_attn2(q, k, v, s):
+    """LightningAttention2 through the native call path where the call has the common form, else through the class."""
+    if s is not None and not torch.compiler.is_compiling():
+        o = _lib.host().attn(q, k, v, s)
+        if o is not None:
+            return o
+    return LightningAttention2.apply(q, k, v, s)
+
+
+def lightning_attn2_no_decay(q, k, v):
+    """LightningAttention2NoDecay, the same way."""
+    if not torch.compiler.is_compiling():
+        o = _lib.host().attn_no_decay(q, k, v)
+        if o is not None:
+            return o
+    return LightningAttention2NoDecay.apply(q, k, v)
+
+
 # The reference's "parallel" variant (lightning_attn2_parallel.py:1072) computes the same function with a
 # different kernel decomposition; here the library picks the decomposition itself.
-lightning_attn2_parallel = LightningAttention2.apply
+lightning_attn2_parallel = lightning_attn2

@@ -88,6 +88,15 @@ class _SrmsNormGate(torch.autograd.Function):
         return dx.reshape(dy.shape), dg.reshape(dy.shape), None
 
 
+def _srms_norm(x, eps):
+    """_SrmsNorm through the native call path (csrc/host_ops.cpp) where the call has the common form, else through the class."""
+    if not torch.compiler.is_compiling():
+        y = _lib.host().norm(x, eps)
+        if y is not None:
+            return y
+    return _SrmsNorm.apply(x, eps)
+
+
 def _aligned16(t):
     """The fused kernels use 128-bit loads: a contiguous view whose storage offset is not 16-byte aligned (a slice of a flat
     buffer) is copied once; fresh allocations are always aligned."""
@@ -104,8 +113,12 @@ def srmsnorm_sigmoid_gate(x, gate, eps=1e-6):
     """SimpleRMSNorm(x) * sigmoid(gate). One fused kernel forward and one backward for rows of up to 16384 16-bit (8192
     fp32) elements that are a multiple of the 128-bit vector width; other rows compose SimpleRMSNorm with torch ops."""
     if _gate_rows_supported(x):
+        if not torch.compiler.is_compiling():
+            y = _lib.host().norm_gate(x, gate, eps)
+            if y is not None:
+                return y
         return _SrmsNormGate.apply(x, gate, eps)
-    return _SrmsNorm.apply(x, eps) * torch.sigmoid(gate)
+    return _srms_norm(x, eps) * torch.sigmoid(gate)
 
 
 class SimpleRMSNorm(torch.nn.Module):
@@ -117,4 +130,4 @@ class SimpleRMSNorm(torch.nn.Module):
         self.dim = dim
 
     def forward(self, x):
-        return _SrmsNorm.apply(x, self.eps)
+        return _srms_norm(x, self.eps)

@@ -38,7 +38,9 @@ def lightning_attn_func(q, k, v, s=None, variant="chunk_loop"):
     """
     if variant not in ("chunk_loop", "parallel"):
         raise ValueError(f"unknown variant {variant!r}")
-    e = v.shape[-1]
+    d, e = q.shape[-1], v.shape[-1]
+    if d % 16 == 0 and e % 16 == 0 and k.shape[-1] == d and d <= _MAX_D and e <= _MAX_D:
+        return lightning_attn2_no_decay(q, k, v) if s is None else lightning_attn2(q, k, v, s)
     q = _pad_last(q, 16)
     k = _pad_last(k, 16)
     v = _pad_last(v, 16)

@@ -1,0 +1,131 @@
+"""The operators' native call path (csrc/host_ops.cpp) against the Python autograd Functions it stands in for."""
+import pytest
+import torch
+
+import lightning_attention_b200 as la
+from lightning_attention_b200 import _lib
+from lightning_attention_b200.ops.cuda.srmsnorm import _SrmsNorm, _SrmsNormGate
+
+DEV = "cuda"
+
+
+def test_cpu_tensors_are_left_to_the_python_operators():
+    x = torch.zeros(1, 2, 16, 16, dtype=torch.bfloat16)
+    H = _lib.host()
+    assert H.attn(x, x, x, torch.zeros(2)) is None and H.attn_no_decay(x, x, x) is None and H.prefill(x, x, x, None, None) is None
+    assert H.decode(x, x, x, None, x) is None and H.norm(x, 1e-6) is None and H.norm_gate(x, x, 1e-6) is None
+    for call in (lambda: la.lightning_attn2(x, x, x, torch.zeros(2)), lambda: la.SimpleRMSNorm(16)(x), lambda: la.srmsnorm_sigmoid_gate(x, x)):
+        with pytest.raises(RuntimeError, match="CUDA tensors only"):
+            call()
+
+
+def _tensors(b, h, n, d, e, bnhd, dtype=torch.bfloat16):
+    torch.manual_seed(31)
+    def one(dim):
+        if bnhd:
+            return torch.randn(b, n, h, dim, device=DEV, dtype=dtype).transpose(1, 2)
+        return torch.randn(b, h, n, dim, device=DEV, dtype=dtype)
+    return [one(d).requires_grad_(), one(d).requires_grad_(), one(e).requires_grad_()], one(e)
+
+
+def _grads(fn, ts, do, **kw):
+    o = fn(*ts)
+    return (o,) + torch.autograd.grad(o, ts, do, **kw)
+
+
+def _same(got, ref):
+    for x, y in zip(got, ref):
+        assert x.shape == y.shape and x.stride() == y.stride() and x.dtype == y.dtype and torch.equal(x, y)
+
+
+SHAPES = [(1, 4, 256, 64, 64, False), (1, 4, 1000, 128, 128, False), (1, 4, 1000, 128, 128, True), (2, 3, 300, 64, 96, True),
+          (4, 32, 130, 128, 128, True), (1, 2, 700, 192, 192, False), (2, 3, 1, 16, 16, False)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,h,n,d,e,bnhd", SHAPES)
+@pytest.mark.parametrize("decay", [True, False])
+def test_attention_equals_the_python_function(cuda_lib, b, h, n, d, e, bnhd, decay):
+    ts, do = _tensors(b, h, n, d, e, bnhd)
+    s = la._build_slope_tensor(h).to(DEV) if decay else None
+    fast = (lambda q, k, v: la.lightning_attn2(q, k, v, s)) if decay else la.lightning_attn2_no_decay
+    slow = (lambda q, k, v: la.LightningAttention2.apply(q, k, v, s)) if decay else la.LightningAttention2NoDecay.apply
+    assert (_lib.host().attn(*ts, s) if decay else _lib.host().attn_no_decay(*ts)) is not None
+    ref = _grads(slow, ts, do)
+    _same(_grads(fast, ts, do), ref)
+    # a gradient in another layout, the graph used twice (kept chunk states, then recomputed ones)
+    odd = do.transpose(2, 3).contiguous().transpose(2, 3)
+    o = fast(*ts)
+    _same(torch.autograd.grad(o, ts, odd, retain_graph=True), ref[1:])
+    for x, y in zip(torch.autograd.grad(o, ts, do), ref[1:]):
+        assert torch.linalg.vector_norm((x - y).float()) <= 1e-2 * torch.linalg.vector_norm(y.float())
+    # saved-tensor hooks: what they return is what the backward pass reads
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(1) or t.clone(), lambda t: t):
+        o = fast(*ts)
+    assert packed
+    _same(torch.autograd.grad(o, ts, do), ref[1:])
+    with torch.no_grad():
+        assert not fast(*ts).requires_grad
+
+
+@pytest.mark.gpu
+def test_other_forms_take_the_python_function(cuda_lib):
+    ts, do = _tensors(1, 4, 200, 64, 64, False)
+    s = la._build_slope_tensor(4).to(DEV)
+    H = _lib.host()
+    odd = [t.detach().transpose(2, 3).contiguous().transpose(2, 3).requires_grad_() for t in ts]
+    assert H.attn(*odd, s) is None and H.attn(*ts, s.cpu()) is None and H.attn(*ts, s.double()) is None
+    ref = _grads(lambda *t: la.lightning_attn2(*t, s), ts, do)
+    _same(_grads(lambda *t: la.lightning_attn2(*t, s.cpu()), odd, do), ref)
+    import torch.autograd.forward_ad as fwAD
+    with fwAD.dual_level():
+        dual = fwAD.make_dual(ts[0].detach(), torch.ones_like(ts[0]))
+        assert H.attn(dual, ts[1], ts[2], s) is None
+        with pytest.raises(RuntimeError):
+            la.lightning_attn2(dual, ts[1], ts[2], s)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda x: la.lightning_attn2(x, x, x, s))(torch.stack([ts[0].detach()] * 2))
+    with pytest.raises(AttributeError):
+        la.lightning_attn2(*ts, None)
+    with pytest.raises(RuntimeError, match="share one dtype"):
+        la.lightning_attn2(ts[0], ts[1].half(), ts[2], s)
+    with pytest.raises(RuntimeError, match="need at least"):
+        la.lightning_attn2(*ts, s[:2])
+    flat = torch.zeros(ts[0].numel() + 1, device=DEV, dtype=torch.bfloat16)[1:].view(ts[0].shape)
+    with pytest.raises(RuntimeError, match="code 6"):
+        la.lightning_attn2(flat, flat, flat, s)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(64,), (5, 33), (3, 7, 512), (2, 4096)])
+def test_norms_equal_the_python_functions(cuda_lib, dtype, shape):
+    torch.manual_seed(32)
+    x, g, dy = (torch.randn(shape, device=DEV, dtype=dtype) for _ in range(3))
+    x.requires_grad_(), g.requires_grad_()
+    assert _lib.host().norm(x, 1e-6) is not None
+    for eps in (1e-6, 1e-3):
+        _same(_grads(lambda t: la.SimpleRMSNorm(shape[-1], eps)(t), [x], dy), _grads(lambda t: _SrmsNorm.apply(t, eps), [x], dy))
+        if shape[-1] % 8 == 0:
+            _same(_grads(lambda t, u: la.srmsnorm_sigmoid_gate(t, u, eps), [x, g], dy), _grads(lambda t, u: _SrmsNormGate.apply(t, u, eps), [x, g], dy))
+    wide = torch.randn(shape + (2,), device=DEV, dtype=dtype)[..., 0]
+    _same(_grads(la.SimpleRMSNorm(shape[-1]), [x], wide), _grads(lambda t: _SrmsNorm.apply(t, 1e-6), [x], wide))
+    assert la.SimpleRMSNorm(shape[-1])(wide).shape == wide.shape
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bnhd", [False, True])
+def test_inference_calls_equal_the_general_product(cuda_lib, bnhd):
+    ts, _ = _tensors(2, 3, 333, 64, 64, bnhd)
+    s = la._build_slope_tensor(3).to(DEV)
+    o, st = la.lightning_attn_prefill(*ts, s)
+    assert not o.requires_grad and _lib.host().prefill(*ts, s, st) is not None
+    _same((o, st), la.la_generic(*[t.detach() for t in ts], s, want_state=True))
+    _same(la.lightning_attn_prefill(*ts, s, st), la.la_generic(*[t.detach() for t in ts], s, state_in=st, want_state=True))
+    q, k, v = (t.detach()[:, :, :1].contiguous() for t in ts)
+    st3, st4 = st.clone(), st.clone()
+    o4 = la.lightning_attn_decode(q, k, v, s, st4)
+    o3 = la.lightning_attn_decode(q[:, :, 0], k[:, :, 0], v[:, :, 0], s.double(), st3)  # fp64 slopes: the Python operator
+    assert o4.shape == v.shape
+    _same((o4[:, :, 0], st4), (o3, st3))
