@@ -88,13 +88,6 @@ bool pick_tiling(int dk, int dv, Tiling* t) {
   return true;
 }
 
-int smem_bytes(int nks, int nvs, int mode, int nstage) {
-  const int slab = LA_SLAB_BYTES;
-  int b = nstage * (nks + 2) * slab;
-  if (mode == 0) b += nks * slab + 2 * slab + nks * nvs * 64 * 128;
-  return b + 64 + 512 + 1024;  // barriers + decay table + alignment slack
-}
-
 int plan_chunks(int bh, int n, int dk, int dv) {
   Tiling t;
   if (!pick_tiling(dk, dv, &t)) return 1;
@@ -110,45 +103,11 @@ int plan_chunks(int bh, int n, int dk, int dv) {
 }
 
 template <int NKS, int NVS, int MODE, int FMT>
-int launch_one(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tC, const LaParams& p, dim3 grid,
-               int smem, cudaStream_t st) {
-  auto kern = la_chunk_kernel<NKS, NVS, MODE, FMT>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
-    cudaGetLastError();
-    return LAB200_ERR_CUDA;
-  }
-  kern<<<grid, LA_THREADS, smem, st>>>(tA, tB, tC, p);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? LAB200_OK : LAB200_ERR_CUDA;
-}
-
-template <int MODE, int FMT>
-int launch_tiled(int nks, int nvs, const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tC,
-                 const LaParams& p, dim3 grid, int smem, cudaStream_t st) {
-#define LAB200_CASE(K, V) \
-  if (nks == K && nvs == V) return launch_one<K, V, MODE, FMT>(tA, tB, tC, p, grid, smem, st);
-  LAB200_CASE(1, 1)
-  LAB200_CASE(1, 2)
-  LAB200_CASE(2, 1)
-  LAB200_CASE(2, 2)
-  LAB200_CASE(3, 1)
-  LAB200_CASE(4, 1)
-#undef LAB200_CASE
-  return LAB200_ERR_SHAPE;
-}
-
-// ---- pipelined kernel (dk <= 128) ---------------------------------------------------------------
-int smem_bytes_pipe(int nks, int nvs, int mode) {
-  const int slab = LA_SLAB_BYTES;
-  int b = 2 * nks * slab + 4 * slab;
-  if (mode == 0) b += 2 * (nks > nvs ? nks : nvs) * slab + nks * nvs * 64 * 128;  // A stages also stage the output tile
-  return b + 2 * LAP_NUM_BARS * 8 + 16 + 512 + 1024;  // barriers, flags, decay table, alignment slack
-}
-
-template <int NKS, int NVS, int MODE, int FMT>
 int launch_pipe_one(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tC, const CUtensorMap& tO,
-                    const LaParams& p, dim3 grid, int smem, cudaStream_t st) {
+                    const LaParams& p, dim3 grid, cudaStream_t st) {
   auto kern = la_pipe_kernel<NKS, NVS, MODE, FMT>;
+  constexpr int smem = lap_smem_bytes(NKS, NVS, MODE);
+  static_assert(smem <= SMEM_LIMIT, "shared memory");
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
     cudaGetLastError();
     return LAB200_ERR_CUDA;
@@ -160,56 +119,28 @@ int launch_pipe_one(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensor
 
 template <int MODE, int FMT>
 int launch_pipe(int nks, int nvs, const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tC,
-                const CUtensorMap& tO, const LaParams& p, dim3 grid, int smem, cudaStream_t st) {
+                const CUtensorMap& tO, const LaParams& p, dim3 grid, cudaStream_t st) {
 #define LAB200_CASE(K, V) \
-  if (nks == K && nvs == V) return launch_pipe_one<K, V, MODE, FMT>(tA, tB, tC, tO, p, grid, smem, st);
+  if (nks == K && nvs == V) return launch_pipe_one<K, V, MODE, FMT>(tA, tB, tC, tO, p, grid, st);
   LAB200_CASE(1, 1)
   LAB200_CASE(1, 2)
   LAB200_CASE(2, 1)
   LAB200_CASE(2, 2)
+  LAB200_CASE(3, 1)
+  LAB200_CASE(4, 1)
 #undef LAB200_CASE
   return LAB200_ERR_SHAPE;
 }
 
-// LIGHTNING_B200_SERIAL=1 in the environment selects the serial block kernel for every shape (A/B comparisons).
-bool use_pipelined_kernel() {
-  static const bool on = [] {
-    const char* e = getenv("LIGHTNING_B200_SERIAL");
-    return !(e && e[0] == '1');
-  }();
-  return on;
-}
-
 int launch_la(int mode, int dtype, const Tiling& t, const CUtensorMap& tA, const CUtensorMap& tB,
-              const CUtensorMap& tC, const CUtensorMap& tO, LaParams p, int nchunks_grid, int bh, cudaStream_t st) {
-  if (t.nks <= 2 && use_pipelined_kernel()) {
-    const int smem = smem_bytes_pipe(t.nks, t.nvs, mode);
-    if (smem <= SMEM_LIMIT) {
-      p.nstage = 2;
-      const dim3 grid(t.nslices, nchunks_grid, bh);
-      if (mode == 0) {
-        return dtype == LAB200_BF16 ? launch_pipe<0, 1>(t.nks, t.nvs, tA, tB, tC, tO, p, grid, smem, st)
-                                    : launch_pipe<0, 0>(t.nks, t.nvs, tA, tB, tC, tO, p, grid, smem, st);
-      }
-      return dtype == LAB200_BF16 ? launch_pipe<1, 1>(t.nks, t.nvs, tA, tB, tC, tO, p, grid, smem, st)
-                                  : launch_pipe<1, 0>(t.nks, t.nvs, tA, tB, tC, tO, p, grid, smem, st);
-    }
-  }
-  int nstage = 2;
-  int smem = smem_bytes(t.nks, t.nvs, mode, nstage);
-  if (smem > SMEM_LIMIT) {
-    nstage = 1;
-    smem = smem_bytes(t.nks, t.nvs, mode, nstage);
-  }
-  if (smem > SMEM_LIMIT) return LAB200_ERR_SHAPE;
-  p.nstage = nstage;
+              const CUtensorMap& tC, const CUtensorMap& tO, const LaParams& p, int nchunks_grid, int bh, cudaStream_t st) {
   const dim3 grid(t.nslices, nchunks_grid, bh);
   if (mode == 0) {
-    return dtype == LAB200_BF16 ? launch_tiled<0, 1>(t.nks, t.nvs, tA, tB, tC, p, grid, smem, st)
-                                : launch_tiled<0, 0>(t.nks, t.nvs, tA, tB, tC, p, grid, smem, st);
+    return dtype == LAB200_BF16 ? launch_pipe<0, 1>(t.nks, t.nvs, tA, tB, tC, tO, p, grid, st)
+                                : launch_pipe<0, 0>(t.nks, t.nvs, tA, tB, tC, tO, p, grid, st);
   }
-  return dtype == LAB200_BF16 ? launch_tiled<1, 1>(t.nks, t.nvs, tA, tB, tC, p, grid, smem, st)
-                              : launch_tiled<1, 0>(t.nks, t.nvs, tA, tB, tC, p, grid, smem, st);
+  return dtype == LAB200_BF16 ? launch_pipe<1, 1>(t.nks, t.nvs, tA, tB, tC, tO, p, grid, st)
+                              : launch_pipe<1, 0>(t.nks, t.nvs, tA, tB, tC, tO, p, grid, st);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -311,14 +242,12 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
   }
 
   LaParams p;
-  p.out = out;
   p.slopes = slopes;
   p.n = n; p.h = h; p.dk = dk; p.dv = dv;
   p.nblocks = nblocks;
   p.blocks_per_chunk = bpc;
   p.reverse = reverse ? 1 : 0;
   p.layout = layout;
-  p.nstage = 2;
   p.wait_budget = WAIT_BUDGET;
   p.trace = g_trace.load(std::memory_order_relaxed);
   p.trace_blocks = g_trace_blocks.load(std::memory_order_relaxed);
@@ -419,7 +348,7 @@ bool use_fused_dkdv() {
     const char* e = getenv("LIGHTNING_B200_FUSED_BWD");
     return !(e && e[0] == '0');
   }();
-  return on && use_pipelined_kernel();
+  return on;
 }
 
 bool dkdv_shape_ok(int d, int e) { return d <= 128 && e <= 128 && (d % 16) == 0 && (e % 16) == 0 && d >= 16 && e >= 16; }
@@ -506,8 +435,8 @@ int la_validate(const void* a, const void* bm, const void* c, const void* out, c
   Tiling t;
   if (bh < 1 || bh > 65535 || h < 1 || n < 1 || !pick_tiling(dk, dv, &t)) return LAB200_ERR_SHAPE;
   // (b, n, h, dim) tensors: whole batches of h heads, third tensor-map coordinate b n h + head within int range, and
-  // only the pipelined kernel (dk <= 128) reads and writes them
-  if (layout && ((bh % h) != 0 || static_cast<long long>(bh) * n >= (1LL << 31) || t.nks > 2 || !use_pipelined_kernel()))
+  // dk <= 128
+  if (layout && ((bh % h) != 0 || static_cast<long long>(bh) * n >= (1LL << 31) || t.nks > 2))
     return LAB200_ERR_SHAPE;
   if (!bm || !c || (!state_only && (!a || !out)) || (state_only == 1 && !state_out)) return LAB200_ERR_SHAPE;
   if (!aligned16(a) || !aligned16(bm) || !aligned16(c) || !aligned16(out) || !aligned16(state_in) ||

@@ -38,7 +38,6 @@ namespace lab200 {
 
 constexpr int LA_BLOCK = 128;        // tokens per block
 constexpr int LA_SLAB_BYTES = 16384; // 128 rows x 128 bytes
-constexpr int LA_THREADS = 256;
 constexpr int LA_TRACE_SLOTS = 16;    // clock stamps per block in the optional trace buffer
 
 enum LaError : int {
@@ -71,7 +70,6 @@ __device__ __forceinline__ void la_status_report(const LaStatus& s, int code) {
 }
 
 struct LaParams {
-  void* out;               // [bh][n][dv], input dtype (unused when only the state is wanted)
   const float* slopes;     // [h] decay rates, or nullptr for no decay
   const float* state_in;   // [bh][state_slots][dv][dk] fp32, or nullptr for a zero initial state
   float* state_out;        // same indexing, or nullptr
@@ -82,9 +80,8 @@ struct LaParams {
   int chunk0;              // chunk handled by blockIdx.y == 0
   int state_slots;         // chunk slots per (batch, head) in state_in / state_out
   int reverse;
-  int layout;              // 0: tensors are (b, h, n, dim) contiguous; 1: (b, n, h, dim) contiguous (pipelined kernel only):
+  int layout;              // 0: tensors are (b, h, n, dim) contiguous; 1: (b, n, h, dim) contiguous:
                            // the tensor maps then index their third dimension by batch * n * h + head, see make_tmap
-  int nstage;              // 1 or 2 shared-memory stages for the Bm and C tiles
   long long wait_budget;   // clock cycles after which a barrier wait gives up
   long long* trace;        // optional: CTA (0,0,0) records clock64() stamps here, LA_TRACE_SLOTS per block
   int trace_blocks;        // capacity of `trace` in blocks
@@ -118,347 +115,6 @@ __device__ __forceinline__ float2 unpack2(uint32_t u) {
   } else {
     return __half22float2(*reinterpret_cast<__half2*>(&u));
   }
-}
-
-// MODE 0: full block loop (writes out, optionally the final state).
-// MODE 1: state only (reads Bm and C, writes the final state).
-// NKS: 64-feature slabs of dk (1..4). NVS: 64-feature slabs of dv handled by this CTA (1..2).
-template <int NKS, int NVS, int MODE, int FMT>
-__global__ void __launch_bounds__(LA_THREADS, 1)
-la_chunk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                const __grid_constant__ CUtensorMap tmC, const LaParams p) {
-  constexpr int SLAB = LA_SLAB_BYTES;
-  constexpr int DV = 64 * NVS;
-  constexpr int DKP = 64 * NKS;
-  constexpr int SC = DKP / 2;  // state columns held per thread
-  constexpr int OC = DV / 2;   // output columns handled per thread
-  constexpr uint32_t T_S = 0, T_OI = 128, T_OX = 128 + DV, T_D = 128 + 2 * DV;
-  static_assert(T_D + DKP <= 512, "TMEM budget");
-  constexpr uint32_t IDESC_S = umma_idesc(FMT, 128, 128, 0, 0);
-  constexpr uint32_t IDESC_X = umma_idesc(FMT, 128, DV, 0, 0);
-  constexpr uint32_t IDESC_PC = umma_idesc(FMT, 128, DV, 0, 1);
-  constexpr uint32_t IDESC_ST = umma_idesc(FMT, 128, DKP, 1, 1);
-
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t base = (raw + 1023u) & ~1023u;
-  const int nstage = p.nstage;
-  const uint32_t sA = base;
-  const uint32_t sB = sA + (MODE == 0 ? NKS * SLAB : 0);
-  const uint32_t sC = sB + nstage * NKS * SLAB;
-  const uint32_t sP = sC + nstage * 2 * SLAB;
-  const uint32_t sS = sP + (MODE == 0 ? 2 * SLAB : 0);
-  const uint32_t sBar = sS + (MODE == 0 ? NKS * DV * 128 : 0);
-  const uint32_t barA = sBar, barBC0 = sBar + 8, barM1 = sBar + 24, barM2 = sBar + 32;
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_raw + (sBar + 40 - raw));
-  // decay table lambda^k, k = 0..127, for the in-block mask (a table look-up per element instead of an
-  // exponential; also keeps the compiler from hoisting 64 exponentials per thread into registers)
-  volatile float* decay_tab = reinterpret_cast<volatile float*>(smem_raw + (sBar + 64 - raw));
-
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
-  const int q = warp & 3, hf = warp >> 2;
-  const int r = q * 32 + lane;  // row inside the block == TMEM lane owned by this thread
-  const uint32_t lanebase = static_cast<uint32_t>(q * 32) << 16;
-
-  const int slice = blockIdx.x;
-  const int chunk = p.chunk0 + blockIdx.y;
-  const int bh = blockIdx.z;
-  const int dv_off = slice * DV;
-  const int blk_begin = chunk * p.blocks_per_chunk;
-  const int blk_end = min(p.nblocks, blk_begin + p.blocks_per_chunk);
-  const int nb = blk_end - blk_begin;
-  const int reverse = p.reverse;
-  const int nk16 = p.dk >> 4;
-
-  la_status_begin(p.status);
-  if (tid == 0) {
-    mbar_init(barA, 1);
-    mbar_init(barBC0, 1);
-    mbar_init(barBC0 + 8, 1);
-    mbar_init(barM1, 1);
-    mbar_init(barM2, 1);
-    fence_mbar_init();
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
-    tma_prefetch_desc(&tmC);
-  }
-  if (warp == 0) {
-    tmem_alloc(sBar + 40, 512);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem = *tmem_slot;
-
-  // per-head decay constants (lightning_attn2.py:41-54)
-  const float s = p.slopes ? p.slopes[bh % p.h] : 0.f;
-  const float s2 = -s * 1.4426950408889634f;  // lambda^x = 2^(s2 x)
-  const float w_fwd = ex2f(s2 * static_cast<float>(r));
-  const float w_bwd = ex2f(s2 * static_cast<float>(LA_BLOCK - r));
-  const float w_out = reverse ? w_bwd : w_fwd;
-  const float w_state = reverse ? w_fwd : w_bwd;
-  const float decay_blk = ex2f(s2 * static_cast<float>(LA_BLOCK));
-  // A forward-time sweep that ends in a ragged block (n not a multiple of 128): the state leaving that block is decayed
-  // to token n, not to the end of the 128-token tile, so that state_out chains exactly (rows >= tail are zero padding).
-  const int tail = p.n - (p.nblocks - 1) * LA_BLOCK;
-  const bool tail_fix = !reverse && tail < LA_BLOCK && blk_end == p.nblocks;
-  const float w_tail = (tail_fix && r < tail) ? ex2f(s2 * static_cast<float>(tail - r)) : 0.f;
-  const float decay_tail = ex2f(s2 * static_cast<float>(tail));
-  if (MODE == 0 && tid < LA_BLOCK) decay_tab[tid] = ex2f(s2 * static_cast<float>(tid));
-
-  auto issue_A = [&](int blk) {
-    mbar_arrive_expect_tx(barA, NKS * SLAB);
-#pragma unroll
-    for (int ks = 0; ks < NKS; ++ks) tma_load_3d(sA + ks * SLAB, &tmA, ks * 64, blk * LA_BLOCK, bh, barA);
-  };
-  auto issue_BC = [&](int blk, int stage) {
-    const uint32_t bar = barBC0 + 8 * stage;
-    mbar_arrive_expect_tx(bar, (NKS + 2) * SLAB);
-#pragma unroll
-    for (int ks = 0; ks < NKS; ++ks)
-      tma_load_3d(sB + (stage * NKS + ks) * SLAB, &tmB, ks * 64, blk * LA_BLOCK, bh, bar);
-#pragma unroll
-    for (int vs = 0; vs < 2; ++vs)
-      tma_load_3d(sC + (stage * 2 + vs) * SLAB, &tmC, dv_off + vs * 64, blk * LA_BLOCK, bh, bar);
-  };
-
-  // first block's loads go out before anything else
-  if (tid == 0 && nb > 0) {
-    const int blk0 = reverse ? (blk_end - 1) : blk_begin;
-    if (MODE == 0) issue_A(blk0);
-    issue_BC(blk0, 0);
-  }
-
-  // running state StateT[j = r][hf * SC .. hf * SC + SC), fp32
-  float st[SC];
-  const bool st_row_valid = (r < DV) && (dv_off + r < p.dv);
-  const bool have_state_in = (p.state_in != nullptr);
-#pragma unroll
-  for (int i = 0; i < SC; ++i) st[i] = 0.f;
-  if (have_state_in && st_row_valid) {
-    const float* src = p.state_in +
-        ((static_cast<size_t>(bh) * p.state_slots + chunk) * p.dv + dv_off + r) * p.dk + hf * SC;
-#pragma unroll
-    for (int i = 0; i < SC; i += 4) {
-      if (hf * SC + i < p.dk) {  // dk is a multiple of 16, so groups of 4 never straddle the edge
-        const float4 v4 = *reinterpret_cast<const float4*>(src + i);
-        st[i] = v4.x; st[i + 1] = v4.y; st[i + 2] = v4.z; st[i + 3] = v4.w;
-      }
-    }
-  }
-  // rounded copy of the state for the tensor cores: K-major B operand, rows = dv index, cols = dk index
-  auto store_state_smem = [&]() {
-    if (r < DV) {
-#pragma unroll
-      for (int i = 0; i < SC; i += 8) {
-        const int col = hf * SC + i;
-        const uint32_t addr = sS + (col >> 6) * (DV * 128) + r * 128 + ((((col & 63) >> 3) ^ (r & 7)) << 4);
-        st_shared_v4(addr, pack2<FMT>(st[i], st[i + 1]), pack2<FMT>(st[i + 2], st[i + 3]),
-                     pack2<FMT>(st[i + 4], st[i + 5]), pack2<FMT>(st[i + 6], st[i + 7]));
-      }
-    }
-  };
-  if (MODE == 0 && have_state_in) {
-    store_state_smem();
-    fence_proxy_async_smem();
-  }
-  __syncthreads();
-
-  int failed = 0;
-  const bool tracing = (p.trace != nullptr) && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
-#define LA_TRACE(slot) if (tracing && it < p.trace_blocks) p.trace[it * LA_TRACE_SLOTS + (slot)] = clock64();
-
-  for (int it = 0; it < nb; ++it) {
-    LA_TRACE(0)
-    const int blk = reverse ? (blk_end - 1 - it) : (blk_begin + it);
-    const int nxt = reverse ? (blk - 1) : (blk + 1);
-    const bool has_next = (it + 1 < nb);
-    const int stage = (nstage == 2) ? (it & 1) : 0;
-    const uint32_t parBC = (nstage == 2) ? ((it >> 1) & 1) : (it & 1);
-    const uint32_t par = it & 1;
-    const uint32_t sBs = sB + stage * NKS * SLAB;
-    const uint32_t sCs = sC + stage * 2 * SLAB;
-    const bool have_state = have_state_in || (it > 0);
-
-    // ---- 1. inputs landed ---------------------------------------------------------------
-    {
-      bool ok = mbar_wait(barBC0 + 8 * stage, parBC, p.wait_budget);
-      if (MODE == 0) ok = ok && mbar_wait(barA, par, p.wait_budget);
-      if (__syncthreads_or(!ok)) { failed = LA_ERR_WAIT_INPUT; break; }
-    }
-    LA_TRACE(1)
-
-    if (MODE == 0) {
-      if (tid == 0) {
-        tc_fence_after_sync();
-        for (int kq = 0; kq < nk16; ++kq) {  // S = A Bm^T
-          const uint32_t off = (kq >> 2) * SLAB + (kq & 3) * 32;
-          umma_f16(tmem + T_S, smem_desc_sw128(sA + off, 16), smem_desc_sw128(sBs + off, 16), IDESC_S, kq > 0);
-        }
-        if (have_state) {
-          for (int kq = 0; kq < nk16; ++kq) {  // O_inter = A State
-            const uint32_t offA = (kq >> 2) * SLAB + (kq & 3) * 32;
-            const uint32_t offS = (kq >> 2) * (DV * 128) + (kq & 3) * 32;
-            umma_f16(tmem + T_OX, smem_desc_sw128(sA + offA, 16), smem_desc_sw128(sS + offS, 16), IDESC_X, kq > 0);
-          }
-        }
-        umma_commit(barM1);
-      }
-      // ---- 2. S ready: mask it into P, scale Bm rows for the state update --------------------
-      {
-        const bool ok = mbar_wait(barM1, par, p.wait_budget);
-        if (__syncthreads_or(!ok)) { failed = LA_ERR_WAIT_MMA1; break; }
-      }
-      LA_TRACE(2)
-      tc_fence_after_sync();
-      if (tid == 0 && has_next) {
-        issue_A(nxt);
-        if (nstage == 2) issue_BC(nxt, stage ^ 1);
-      }
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c0 = hf * 64 + cc * 32;
-        // warp-uniform: is this 32x32 tile entirely on the masked side?
-        const bool dead = reverse ? (c0 + 31 < q * 32) : (c0 > q * 32 + 31);
-        uint32_t v[32];
-        if (!dead) {
-          tmem_ld32(tmem + lanebase + T_S + c0, v);
-          tmem_wait_ld();
-        }
-        uint32_t pk[16];
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float f0 = 0.f, f1 = 0.f;
-          if (!dead) {
-            const int d0 = reverse ? (c0 + i - r) : (r - c0 - i);  // distance on the causal side when >= 0
-            const int d1 = reverse ? (d0 + 1) : (d0 - 1);
-            if (d0 >= 0) f0 = __uint_as_float(v[i]) * decay_tab[d0];
-            if (d1 >= 0) f1 = __uint_as_float(v[i + 1]) * decay_tab[d1];
-          }
-          pk[i >> 1] = pack2<FMT>(f0, f1);
-        }
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const uint32_t addr = sP + hf * SLAB + r * 128 + (((cc * 4 + g) ^ (r & 7)) << 4);
-          st_shared_v4(addr, pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
-        }
-      }
-    } else {
-      if (tid == 0 && has_next && nstage == 2) issue_BC(nxt, stage ^ 1);
-    }
-
-    // Bm rows *= w_state(r), in place (the S MMA no longer needs the unscaled tile)
-    const bool tail_blk = tail_fix && it == nb - 1;
-    const float w_st = tail_blk ? w_tail : w_state;
-#pragma unroll
-    for (int i = 0; i < NKS * 4; ++i) {
-      const int g = hf * NKS * 4 + i;
-      const int ks = g >> 3, p0 = g & 7;
-      const int pos = (p0 & 4) | ((p0 + r) & 3);
-      const uint32_t addr = sBs + ks * SLAB + r * 128 + (pos << 4);
-      uint32_t u0, u1, u2, u3;
-      ld_shared_v4(addr, u0, u1, u2, u3);
-      float2 f;
-      f = unpack2<FMT>(u0); u0 = pack2<FMT>(f.x * w_st, f.y * w_st);
-      f = unpack2<FMT>(u1); u1 = pack2<FMT>(f.x * w_st, f.y * w_st);
-      f = unpack2<FMT>(u2); u2 = pack2<FMT>(f.x * w_st, f.y * w_st);
-      f = unpack2<FMT>(u3); u3 = pack2<FMT>(f.x * w_st, f.y * w_st);
-      st_shared_v4(addr, u0, u1, u2, u3);
-    }
-    fence_proxy_async_smem();
-    tc_fence_before_sync();
-    __syncthreads();
-    LA_TRACE(3)
-
-    // ---- 3. O_intra = P C ; StateT_local = C^T (w_state Bm) ------------------------------------
-    if (tid == 0) {
-      tc_fence_after_sync();
-      if (MODE == 0) {
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          umma_f16(tmem + T_OI, smem_desc_sw128(sP + (kk >> 2) * SLAB + (kk & 3) * 32, 16),
-                   smem_desc_sw128(sCs + kk * 2048, SLAB), IDESC_PC, kk > 0);
-        }
-      }
-#pragma unroll
-      for (int kk = 0; kk < 8; ++kk) {
-        umma_f16(tmem + T_D, smem_desc_sw128(sCs + kk * 2048, SLAB), smem_desc_sw128(sBs + kk * 2048, SLAB),
-                 IDESC_ST, kk > 0);
-      }
-      umma_commit(barM2);
-    }
-    {
-      const bool ok = mbar_wait(barM2, par, p.wait_budget);
-      if (__syncthreads_or(!ok)) { failed = LA_ERR_WAIT_MMA2; break; }
-    }
-    LA_TRACE(4)
-    tc_fence_after_sync();
-    if (tid == 0 && has_next && nstage == 1) issue_BC(nxt, 0);
-
-    // ---- 4. epilogue: out rows, then the state recurrence ---------------------------------------
-    if (MODE == 0) {
-      const int tok = blk * LA_BLOCK + r;
-#pragma unroll
-      for (int cc = 0; cc < OC; cc += 32) {
-        uint32_t a[32], b[32];
-        tmem_ld32(tmem + lanebase + T_OI + hf * OC + cc, a);
-        if (have_state) tmem_ld32(tmem + lanebase + T_OX + hf * OC + cc, b);
-        tmem_wait_ld();
-        if (tok < p.n) {
-          const int col0 = dv_off + hf * OC + cc;
-          uint8_t* orow = static_cast<uint8_t*>(p.out) + ((static_cast<size_t>(bh) * p.n + tok) * p.dv + col0) * 2;
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            if (col0 + g * 8 < p.dv) {
-              uint32_t o4[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float x0 = __uint_as_float(a[g * 8 + 2 * j]), x1 = __uint_as_float(a[g * 8 + 2 * j + 1]);
-                if (have_state) {
-                  x0 = fmaf(w_out, __uint_as_float(b[g * 8 + 2 * j]), x0);
-                  x1 = fmaf(w_out, __uint_as_float(b[g * 8 + 2 * j + 1]), x1);
-                }
-                o4[j] = pack2<FMT>(x0, x1);
-              }
-              *reinterpret_cast<uint4*>(orow + g * 16) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
-            }
-          }
-        }
-      }
-    }
-    if (q * 32 < DV) {  // warp-uniform: lanes >= DV of the state accumulator hold nothing useful
-#pragma unroll
-      for (int cc = 0; cc < SC; cc += 32) {
-        uint32_t dl[32];
-        tmem_ld32(tmem + lanebase + T_D + hf * SC + cc, dl);
-        tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) st[cc + i] = fmaf(tail_blk ? decay_tail : decay_blk, st[cc + i], __uint_as_float(dl[i]));
-      }
-      if (MODE == 0 && has_next) store_state_smem();
-    }
-    fence_proxy_async_smem();
-    tc_fence_before_sync();
-    __syncthreads();
-    LA_TRACE(5)
-  }
-#undef LA_TRACE
-
-  if (!failed && p.state_out != nullptr && st_row_valid) {
-    float* dst = p.state_out +
-        ((static_cast<size_t>(bh) * p.state_slots + chunk) * p.dv + dv_off + r) * p.dk + hf * SC;
-#pragma unroll
-    for (int i = 0; i < SC; i += 4) {
-      if (hf * SC + i < p.dk) *reinterpret_cast<float4*>(dst + i) = make_float4(st[i], st[i + 1], st[i + 2], st[i + 3]);
-    }
-  }
-  if (failed && tid == 0) la_status_report(p.status, failed);
-
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 // Exclusive decayed scan over the per-chunk local states, in place:

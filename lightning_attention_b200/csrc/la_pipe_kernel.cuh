@@ -1,9 +1,6 @@
-// Warp-specialised, software-pipelined version of the Lightning Attention-2 block kernel (dk <= 128).
-//
-// Same mathematics, operands, shared-memory slab layout and state conventions as la_chunk_kernel in
-// la_kernels.cuh; what changes is who does what and when. The serial kernel runs the phases of one
-// 128-token block one after another behind CTA-wide barriers; here four roles work on different blocks
-// at the same time and hand tiles to each other through mbarriers:
+// The Lightning Attention-2 block kernel: warp-specialised and software-pipelined. Mathematics, operands, shared-memory slab layout
+// and state conventions are described in la_kernels.cuh. Four roles work on different 128-token blocks at the same time and hand
+// tiles to each other through mbarriers:
 //
 //   warp 0      TMA producer   loads A, Bm, C tiles of block i+1, i+2 into two shared-memory stages
 //   warp 1      MMA issuer     X_i = A State_i, D_i = C^T (w Bm), PC_i = P_i C, S_{i+1} = A Bm^T, in this order (one thread)
@@ -14,6 +11,15 @@
 // P never touches shared memory: it is written to TMEM with tcgen05.st and consumed by tcgen05.mma as the
 // A operand, which frees the 32 KB that double-buffering A needs. Every wait is bounded and checks a
 // CTA-wide abort flag, so a protocol error ends with an error status instead of a hang.
+//
+// Key widths of 129 to 256 (NKS = 3, 4; WIDE) run the same roles on 64-wide dv slices, with two differences. What does not fit twice
+// into 227 KB has one stage: A always (200 KB at NKS = 3), at NKS = 4 Bm too; A is reloaded as soon as X_i has read it. And the
+// fp32 state is held un-transposed: a warp can only read the TMEM lanes of its own quadrant, and the accumulator C^T (w Bm) has dv
+// on its lanes, so with a 64-wide slice half of the state warps would reach nothing and the others need 96 to 128 registers per
+// thread for their share. (w Bm)^T C has dk on its lanes, two M = 128 tiles of 64 columns, one per half of the state group: 64
+// registers per thread, and the copy X reads is then a [dk][64] slab used as an MN-major operand, like C itself. What bounds a
+// block is the chain X_i -> reload of A -> S_{i+1} -> mask -> P C. b2 h12 n2048 d=e=192: 59.6 us per launch with the phases of a
+// block one after another behind CTA-wide barriers (the kernel these widths had before), now 31.8 (state-only pass 25.0 -> 17.7).
 #pragma once
 #include "la_kernels.cuh"
 
@@ -25,7 +31,18 @@ constexpr int LAP_MASK_THREADS = 128, LAP_STATE_THREADS = 256;
 
 // barrier slots (each has two instances, indexed by block parity)
 enum : int { LAP_FULL_AB = 0, LAP_FULL_C, LAP_S_READY, LAP_P_READY, LAP_PC_DONE, LAP_D_DONE, LAP_O_FREE, LAP_D_FREE,
-             LAP_STATE_READY, LAP_O_STAGED, LAP_BM_SCALED, LAP_NUM_BARS };
+             LAP_STATE_READY, LAP_O_STAGED, LAP_BM_SCALED, LAP_A_FREE, LAP_NUM_BARS };
+
+// Shared-memory stages, in 16 KB slabs (host and device agree through these).
+__host__ __device__ constexpr bool lap_wide(int nks) { return nks > 2; }
+__host__ __device__ constexpr int lap_a_slabs(int nks, int nvs) { return lap_wide(nks) ? nks : 2 * (nks > nvs ? nks : nvs); }  // all stages of A, full block loop
+__host__ __device__ constexpr int lap_b_stages(int nks, int mode) { return (nks == 4 && mode == 0) ? 1 : 2; }
+__host__ __device__ constexpr int lap_c_slabs(int nks) { return lap_wide(nks) ? 1 : 2; }  // per stage: the M = 128 side of D for dk <= 128 reads two
+__host__ __device__ constexpr int lap_smem_bytes(int nks, int nvs, int mode) {
+  int b = (lap_b_stages(nks, mode) * nks + 2 * lap_c_slabs(nks)) * LA_SLAB_BYTES;
+  if (mode == 0) b += lap_a_slabs(nks, nvs) * LA_SLAB_BYTES + nks * nvs * 64 * 128;
+  return b + 2 * LAP_NUM_BARS * 8 + 16 + 512 + 1024;  // barriers, flags, decay table, alignment slack
+}
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -64,27 +81,33 @@ template <int NKS, int NVS, int MODE, int FMT>
 __global__ void __launch_bounds__(LAP_THREADS, 1)
 la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmO, const LaParams p) {
-  static_assert(NKS <= 2, "the pipelined kernel double-buffers all inputs; dk <= 128 only");
+  constexpr bool WIDE = lap_wide(NKS);
+  static_assert(NKS <= 4 && NVS <= 2 && (!WIDE || NVS == 1), "tile sizes");
   constexpr int SLAB = LA_SLAB_BYTES;
   constexpr int DV = 64 * NVS;
   constexpr int DKP = 64 * NKS;
-  constexpr int SC = DKP / 2;
+  constexpr int SC = WIDE ? DV : DKP / 2;  // state columns per thread
   constexpr int OC = DV / 2;
-  constexpr int NAS = NKS > NVS ? NKS : NVS;  // slabs per A stage: the stage also stages the block's output tile
+  constexpr int NAS = WIDE ? 0 : (NKS > NVS ? NKS : NVS);  // slabs from one A stage to the next (0: there is one)
+  constexpr int NBS = lap_b_stages(NKS, MODE) == 2 ? NKS : 0;
+  constexpr int NCS = lap_c_slabs(NKS);
   constexpr uint32_t T_S = 0, T_OI = 128, T_OX = 128 + DV, T_D = 128 + 2 * DV;
-  static_assert(T_D + DKP <= 512, "TMEM budget");
+  static_assert(T_D + (WIDE ? 2 * DV : DKP) <= 512, "TMEM budget");
   constexpr uint32_t IDESC_S = umma_idesc(FMT, 128, 128, 0, 0);
   constexpr uint32_t IDESC_X = umma_idesc(FMT, 128, DV, 0, 0);
   constexpr uint32_t IDESC_PC = umma_idesc(FMT, 128, DV, 0, 1);
-  constexpr uint32_t IDESC_ST = umma_idesc(FMT, 128, DKP, 1, 1);
+  constexpr uint32_t IDESC_ST = umma_idesc(FMT, 128, WIDE ? DV : DKP, 1, 1);
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
-  const uint32_t sA = base;                                         // 2 stages x NAS slabs (MODE 0)
-  const uint32_t sB = sA + (MODE == 0 ? 2 * NAS * SLAB : 0);        // 2 stages x NKS slabs
-  const uint32_t sC = sB + 2 * NKS * SLAB;                          // 2 stages x 2 slabs
-  const uint32_t sS = sC + 2 * 2 * SLAB;                            // bf16 state, NKS x [DV rows][128 B] (MODE 0)
+  const uint32_t sA = base;                                         // 2 stages x NAS slabs, wide: 1 x NKS (MODE 0)
+  const uint32_t sB = sA + (MODE == 0 ? lap_a_slabs(NKS, NVS) * SLAB : 0);  // 2 stages x NKS slabs (NKS = 4, MODE 0: 1)
+  const uint32_t sC = sB + lap_b_stages(NKS, MODE) * NKS * SLAB;    // 2 stages x NCS slabs
+  // 16-bit state: NKS x [DV rows][128 B] (rows dv, columns dk); wide: [DKP rows][128 B] (rows dk, columns dv) (MODE 0). The second
+  // M = 128 tile of D at NKS = 3 reads one slab behind its Bm stage: that is the other stage or C, and only reaches accumulator
+  // rows that nobody reads.
+  const uint32_t sS = sC + 2 * NCS * SLAB;
   // Output tiles are staged in the C stage of their own block (free once P C is done) and leave by TMA store.
   const uint32_t sBar = sS + (MODE == 0 ? NKS * DV * 128 : 0);      // 2 x LAP_NUM_BARS mbarriers
   const uint32_t sMisc = sBar + 2 * LAP_NUM_BARS * 8;
@@ -154,7 +177,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (!lap_wait(bar(LAP_O_STAGED, sst), (i >> 1) & 1, abort_flag, budget)) return false;
 #pragma unroll
         for (int vs = 0; vs < NVS; ++vs)
-          tma_store_3d(&tmO, sC + (sst * 2 + vs) * SLAB, dv_off + vs * 64, blk_of(i) * LA_BLOCK, zc);
+          tma_store_3d(&tmO, sC + (sst * NCS + vs) * SLAB, dv_off + vs * 64, blk_of(i) * LA_BLOCK, zc);
         tma_store_commit();
         return true;
       };
@@ -165,17 +188,27 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const uint32_t prev_par = ((it >> 1) & 1) ^ 1;  // parity of the previous use of this stage (block it-2)
         // A and Bm of block it: their stages are free once every MMA of block it-2 has run (P C is the last one issued; in
         // state-only mode D). They are what S of block it waits for, so they go first and wait for nothing else.
-        if (it >= 2) {
+        // Where there is one stage, A is free after X of block it-1 and Bm after D of block it-1.
+        const uint32_t last_par = ((it - 1) >> 1) & 1;
+        auto load_b = [&]() {
+#pragma unroll
+          for (int ks = 0; ks < NKS; ++ks)
+            tma_load_3d(sB + (st * NBS + ks) * SLAB, &tmB, ks * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_AB, st));
+        };
+        if (NBS != 0 && it >= 2) {
           if (!lap_wait(bar(MODE == 0 ? LAP_PC_DONE : LAP_D_DONE, st), prev_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
         }
         mbar_arrive_expect_tx(bar(LAP_FULL_AB, st), (MODE == 0 ? 2 * NKS : NKS) * SLAB);
-#pragma unroll
-        for (int ks = 0; ks < NKS; ++ks)
-          tma_load_3d(sB + (st * NKS + ks) * SLAB, &tmB, ks * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_AB, st));
+        if (NBS != 0) load_b();
         if (MODE == 0) {
+          if (NAS == 0 && it >= 1 && !lap_wait(bar(LAP_A_FREE, st ^ 1), last_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
 #pragma unroll
           for (int ks = 0; ks < NKS; ++ks)
             tma_load_3d(sA + (st * NAS + ks) * SLAB, &tmA, ks * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_AB, st));
+        }
+        if (NBS == 0) {
+          if (it >= 1 && !lap_wait(bar(LAP_D_DONE, st ^ 1), last_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+          load_b();
         }
         // C of block it: in the full block loop its stage holds the staged output tile of block it-2, which is stored first;
         // C is not needed before D of block it, a whole block later than A and Bm.
@@ -188,7 +221,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         mbar_arrive_expect_tx(bar(LAP_FULL_C, st), NVS * SLAB);
 #pragma unroll
         for (int vs = 0; vs < NVS; ++vs)
-          tma_load_3d(sC + (st * 2 + vs) * SLAB, &tmC, dv_off + vs * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_C, st));
+          tma_load_3d(sC + (st * NCS + vs) * SLAB, &tmC, dv_off + vs * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_C, st));
       }
       if (MODE == 0 && alive && *abort_flag == 0) {
         for (int i = max(nb - 2, 0); i < nb; ++i) {
@@ -209,7 +242,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int ist = i & 1;
         if (!lap_wait(bar(LAP_FULL_AB, ist), (i >> 1) & 1, abort_flag, budget)) return false;
         tc_fence_after_sync();
-        const uint32_t a0 = sA + ist * NAS * SLAB, b0 = sB + ist * NKS * SLAB;
+        const uint32_t a0 = sA + ist * NAS * SLAB, b0 = sB + ist * NBS * SLAB;
         for (int kq = 0; kq < nk16; ++kq) {  // S = A Bm^T
           const uint32_t off = (kq >> 2) * SLAB + (kq & 3) * 32;
           umma_f16(tmem + T_S, smem_desc_sw128(a0 + off, 16), smem_desc_sw128(b0 + off, 16), IDESC_S, kq > 0);
@@ -227,7 +260,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const uint32_t par = (it >> 1) & 1;
         const int pst = st ^ 1;                         // instance used by block it-1
         const uint32_t ppar = ((it - 1) >> 1) & 1;      // and its parity
-        const uint32_t sAs = sA + st * NAS * SLAB, sBs = sB + st * NKS * SLAB, sCs = sC + st * 2 * SLAB;
+        const uint32_t sAs = sA + st * NAS * SLAB, sBs = sB + st * NBS * SLAB, sCs = sC + st * NCS * SLAB;
         const bool have_state = have_state_in || (it > 0);
         LAP_TRACE(0, it)
         if (MODE == 0) {
@@ -237,10 +270,15 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             tc_fence_after_sync();
             for (int kq = 0; kq < nk16; ++kq) {  // X = A State
               const uint32_t offA = (kq >> 2) * SLAB + (kq & 3) * 32;
-              const uint32_t offS = (kq >> 2) * (DV * 128) + (kq & 3) * 32;
-              umma_f16(tmem + T_OX, smem_desc_sw128(sAs + offA, 16), smem_desc_sw128(sS + offS, 16), IDESC_X, kq > 0);
+              if constexpr (WIDE) {
+                umma_f16(tmem + T_OX, smem_desc_sw128(sAs + offA, 16), smem_desc_sw128(sS + kq * 2048, SLAB), IDESC_PC, kq > 0);
+              } else {
+                const uint32_t offS = (kq >> 2) * (DV * 128) + (kq & 3) * 32;
+                umma_f16(tmem + T_OX, smem_desc_sw128(sAs + offA, 16), smem_desc_sw128(sS + offS, 16), IDESC_X, kq > 0);
+              }
             }
           }
+          if (WIDE) umma_commit(bar(LAP_A_FREE, st));  // S and X of this block are done with A
           LAP_TRACE(1, it)
         }
         if (MODE != 0 && !lap_wait(bar(LAP_FULL_AB, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_INPUT) break; }
@@ -248,9 +286,16 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (!lap_wait(bar(LAP_BM_SCALED, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
         if (it > 0 && !lap_wait(bar(LAP_D_FREE, pst), ppar, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
         tc_fence_after_sync();
+        if constexpr (WIDE) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)  // local StateT = C^T (w_state Bm)
-          umma_f16(tmem + T_D, smem_desc_sw128(sCs + kk * 2048, SLAB), smem_desc_sw128(sBs + kk * 2048, SLAB), IDESC_ST, kk > 0);
+          for (int kk = 0; kk < 16; ++kk)  // local State = (w_state Bm)^T C, dk rows 0-127 and 128-255
+            umma_f16(tmem + T_D + (kk >> 3) * DV, smem_desc_sw128(sBs + (kk >> 3) * 2 * SLAB + (kk & 7) * 2048, SLAB),
+                     smem_desc_sw128(sCs + (kk & 7) * 2048, SLAB), IDESC_ST, (kk & 7) > 0);
+        } else {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)  // local StateT = C^T (w_state Bm)
+            umma_f16(tmem + T_D, smem_desc_sw128(sCs + kk * 2048, SLAB), smem_desc_sw128(sBs + kk * 2048, SLAB), IDESC_ST, kk > 0);
+        }
         umma_commit(bar(LAP_D_DONE, st));  // also: X_it is done with the bf16 state copy
         LAP_TRACE(3, it)
         if (MODE == 0) {
@@ -361,29 +406,39 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const float w_tail = (tail_fix && r < tail) ? ex2f(s2 * static_cast<float>(tail - r)) : 0.f;
     const uint32_t w_tail2 = pack2<FMT>(w_tail, w_tail);
     const float decay_tail = ex2f(s2 * static_cast<float>(tail));
-    const bool st_row_valid = (r < DV) && (dv_off + r < p.dv);
+    // this thread's part of the state: row r (dv), columns hf SC + i (dk); wide: row hf 128 + r (dk), columns i (dv)
+    const int st_row = WIDE ? hf * 128 + r : r;
+    const bool st_warp = WIDE ? (hf * 128 + q * 32 < DKP) : (q * 32 < DV);  // the accumulator lanes of this warp hold state rows
+    const bool st_row_valid = WIDE ? (st_row < p.dk) : ((r < DV) && (dv_off + r < p.dv));
     const bool store_thread = (w8 == 0 && lane == 0);
 
     float stt[SC];
 #pragma unroll
     for (int i = 0; i < SC; ++i) stt[i] = 0.f;
     if (have_state_in && st_row_valid) {
-      const float* src = p.state_in +
-          ((static_cast<size_t>(bh) * p.state_slots + chunk) * p.dv + dv_off + r) * p.dk + hf * SC;
+      const float* src = p.state_in + (static_cast<size_t>(bh) * p.state_slots + chunk) * p.dv * p.dk;
+      if constexpr (WIDE) {  // neighbouring lanes read neighbouring dk
+        src += static_cast<size_t>(dv_off) * p.dk + st_row;
 #pragma unroll
-      for (int i = 0; i < SC; i += 4) {
-        if (hf * SC + i < p.dk) {
-          const float4 v4 = *reinterpret_cast<const float4*>(src + i);
-          stt[i] = v4.x; stt[i + 1] = v4.y; stt[i + 2] = v4.z; stt[i + 3] = v4.w;
+        for (int i = 0; i < SC; ++i)
+          if (dv_off + i < p.dv) stt[i] = src[static_cast<size_t>(i) * p.dk];
+      } else {
+        src += static_cast<size_t>(dv_off + r) * p.dk + hf * SC;
+#pragma unroll
+        for (int i = 0; i < SC; i += 4) {
+          if (hf * SC + i < p.dk) {
+            const float4 v4 = *reinterpret_cast<const float4*>(src + i);
+            stt[i] = v4.x; stt[i + 1] = v4.y; stt[i + 2] = v4.z; stt[i + 3] = v4.w;
+          }
         }
       }
     }
     auto store_state_smem = [&]() {
-      if (r < DV) {
+      if (WIDE ? st_warp : (r < DV)) {
 #pragma unroll
         for (int i = 0; i < SC; i += 8) {
-          const int col = hf * SC + i;
-          const uint32_t addr = sS + (col >> 6) * (DV * 128) + r * 128 + ((((col & 63) >> 3) ^ (r & 7)) << 4);
+          const int col = WIDE ? i : hf * SC + i;
+          const uint32_t addr = sS + (col >> 6) * (DV * 128) + st_row * 128 + ((((col & 63) >> 3) ^ (r & 7)) << 4);
           st_shared_v4(addr, pack2<FMT>(stt[i], stt[i + 1]), pack2<FMT>(stt[i + 2], stt[i + 3]),
                        pack2<FMT>(stt[i + 4], stt[i + 5]), pack2<FMT>(stt[i + 6], stt[i + 7]));
         }
@@ -404,10 +459,31 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       bool ok = lap_wait(bar(MODE == 0 ? LAP_S_READY : LAP_FULL_AB, st), (j >> 1) & 1, abort_flag, budget);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) return false;
-      if (s != 0.f) {
+      if (WIDE && s != 0.f) {
+        // w in fp32 here: one rounding per element; two slabs at a time keep the registers in bounds
+        const float w = (tail_fix && j == nb - 1) ? w_tail : w_state;
+        const uint32_t row = sB + st * NBS * SLAB + r * 128;
+#pragma unroll 1
+        for (int ks = 0; ks < NKS; ++ks) {
+          uint32_t u[4][4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c)  // positions rotate with the row: eight rows cover all banks
+            ld_shared_v4(row + ks * SLAB + (((hf * 4 + c + r) & 7) << 4), u[c][0], u[c][1], u[c][2], u[c][3]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+#pragma unroll
+            for (int j2 = 0; j2 < 4; ++j2) {
+              const float2 f = unpack2<FMT>(u[c][j2]);
+              u[c][j2] = pack2<FMT>(f.x * w, f.y * w);
+            }
+            st_shared_v4(row + ks * SLAB + (((hf * 4 + c + r) & 7) << 4), u[c][0], u[c][1], u[c][2], u[c][3]);
+          }
+        }
+        fence_proxy_async_smem();
+      } else if (!WIDE && s != 0.f) {
         const uint32_t w2 = (tail_fix && j == nb - 1) ? w_tail2 : w_state2;
         constexpr int NCH = NKS * 4;  // chunks per thread
-        const uint32_t sBs = sB + st * NKS * SLAB;
+        const uint32_t sBs = sB + st * NBS * SLAB;
         uint32_t u[NCH][4];
         uint32_t addr[NCH];
 #pragma unroll
@@ -452,7 +528,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (store_thread) { LAP_TRACE(8, it) }
       tc_fence_after_sync();
       // ---- state recurrence --------------------------------------------------------------------------
-      if (q * 32 < DV) {
+      if (st_warp) {
 #pragma unroll
         for (int cc = 0; cc < SC; cc += 32) {
           uint32_t dl[32];
@@ -480,7 +556,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (!ok) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
         if (store_thread) { LAP_TRACE(7, it) }
         tc_fence_after_sync();
-        const uint32_t sOs = sC + st * 2 * SLAB;  // P C and D of this block are done with this C stage
+        const uint32_t sOs = sC + st * NCS * SLAB;  // P C and D of this block are done with this C stage
 #pragma unroll
         for (int cc = 0; cc < OC; cc += 16) {
           uint32_t a[16], b[16];
@@ -515,11 +591,18 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (MODE == 0 && has_next && !scale_bm(it + 1)) { LAP_FAIL(LA_ERR_WAIT_MMA1) break; }
     }
     if (*abort_flag == 0 && p.state_out != nullptr && st_row_valid) {
-      float* dst = p.state_out +
-          ((static_cast<size_t>(bh) * p.state_slots + chunk) * p.dv + dv_off + r) * p.dk + hf * SC;
+      float* dst = p.state_out + (static_cast<size_t>(bh) * p.state_slots + chunk) * p.dv * p.dk;
+      if constexpr (WIDE) {
+        dst += static_cast<size_t>(dv_off) * p.dk + st_row;
 #pragma unroll
-      for (int i = 0; i < SC; i += 4) {
-        if (hf * SC + i < p.dk) *reinterpret_cast<float4*>(dst + i) = make_float4(stt[i], stt[i + 1], stt[i + 2], stt[i + 3]);
+        for (int i = 0; i < SC; ++i)
+          if (dv_off + i < p.dv) dst[static_cast<size_t>(i) * p.dk] = stt[i];
+      } else {
+        dst += static_cast<size_t>(dv_off + r) * p.dk + hf * SC;
+#pragma unroll
+        for (int i = 0; i < SC; i += 4) {
+          if (hf * SC + i < p.dk) *reinterpret_cast<float4*>(dst + i) = make_float4(stt[i], stt[i + 1], stt[i + 2], stt[i + 3]);
+        }
       }
     }
   }

@@ -520,6 +520,33 @@ def test_prefill_chunks_and_decode_steps_continue_the_sequence(cuda_lib, d, e, d
     assert O.rel_l2_err(f(st), O.state_entering(f(k), f(v), f(s))) <= 1e-2
 
 
+@pytest.mark.parametrize("n,dk,dv,chunks", [(1, 144, 16, 1), (127, 144, 64, 1), (129, 192, 80, 1), (513, 192, 192, 2), (640, 208, 64, 1),
+                                            (700, 256, 256, 1), (1025, 256, 48, 3), (900, 176, 320, 2)])
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 5e-3), (torch.float16, 7e-4)])
+def test_wide_keys_against_the_oracle(cuda_lib, n, dk, dv, chunks, reverse, dtype, tol):
+    """129 <= dk <= 256: single-staged A (and, from 193 on, Bm), dk on the lanes of the state accumulator. One block to several,
+    both directions, widths that end inside a slab, an incoming state, the state alone. Scores, scaled Bm, state copy and result are
+    each rounded once to the 16-bit type (relative 2^-9 or 2^-12 at most, 0.58 of that rms): below 4 * 0.58 * 2^-9 = 4.5e-3 or 5.7e-4."""
+    torch.manual_seed(41)
+    b, h = 2, 3
+    a, bm = (0.5 * torch.randn((b, h, n, dk), device=DEV).to(dtype) for _ in range(2))
+    c = torch.randn((b, h, n, dv), device=DEV).to(dtype)
+    s = la._build_slope_tensor(h).reshape(-1).to(DEV)
+    s[1] = 0.004
+    s[2] = 0.0
+    f = lambda t: None if t is None else t.double().cpu().numpy()
+    for st_in in (None, torch.randn((b, h, dv, dk), device=DEV) if not reverse or n % 128 == 0 else None):
+        out, st = c_generic(cuda_lib, a, bm, c, s, reverse, st_in, True, chunks)
+        ref, ref_st = O.la_generic(f(a), f(bm), f(c), f(s), reverse=reverse, state_in=f(st_in))
+        assert O.rel_l2_err(f(out), ref) <= tol
+        if not reverse:
+            want = O.state_entering(f(bm), f(c), f(s), state_in=f(st_in))
+            assert O.rel_l2_err(f(st), want) <= tol
+            only = c_generic(cuda_lib, None, bm, c, s, reverse, st_in, True, chunks, state_only=True)[1]
+            assert O.rel_l2_err(f(only), want) <= tol
+
+
 def test_decode_step_against_numpy_oracle(cuda_lib):
     torch.manual_seed(23)
     b, h, d, e = 3, 5, 48, 80
