@@ -25,10 +25,10 @@
 //   q: load -> S1, P0 q (commit QP_DONE) -> rows scaled in place (state group) -> D (commit D_DONE) -> next load
 //   k: load -> S1 -> mask pass 1 -> scaled copy Ks, by the same warps (PK1_READY) -> next load
 //   v: load -> S0 (issued one block ahead) -> mask pass 0 -> scaled copy Vs (PV0_READY) -> next load
-// Roles (480 threads): warp 0 issues the loads, in the order in which their buffers come free; warp 1 issues the MMAs (one
-// elected thread), per block: P0 q | Vs dKV^T | S0 of the next block | D | P1 do + Ks dKV | S1 of the next block; warps 2-5
+// Roles (512 threads): warp 0 issues the loads, in the order in which their buffers come free; warp 1 issues the MMAs (one
+// elected thread), per block: P0 q | Vs dKV^T | S0 of the next block | D | P1 do + Ks dKV | S1 of the next block; warps 4-7
 // are the mask group (one per TMEM lane quadrant), which also writes the scaled copies right behind its own mask passes;
-// warps 6-13 are the state/output group (q scaling, the two output tiles, the state recurrence and its bf16 copy); warp 14
+// warps 8-15 are the state/output group (q scaling, the two output tiles, the state recurrence and its bf16 copy); warp 2
 // stores the staged output tiles, so that waiting for a store to have read the staging buffer never delays a load.
 // Every wait is bounded and polls a CTA-wide abort flag.
 #pragma once
@@ -51,7 +51,11 @@ struct LaDkdvParams {
   int trace_blocks;
 };
 
-constexpr int LD2_THREADS = 480;  // 15 warps: 65536 / 480 still allows 128 registers per thread
+// Warpgroups and register split as in la_pipe_kernel.cuh; here the 128 registers of an even split spilled 36 bytes:
+// b2 h16 n4096 d=e=128 backward 130.5 -> 124.7 us, b4 h32 n32768 2045 -> 2000.
+constexpr int LD2_THREADS = 512;
+constexpr int LD2_REGS[3] = {96, 128, 144};
+static_assert(LD2_REGS[0] + LD2_REGS[1] + 2 * LD2_REGS[2] <= 512, "the split must not ask for more than the launch gave");
 
 // barrier slots; every slot has two instances indexed by block parity
 enum : int {
@@ -146,7 +150,7 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #ifdef LD2_WAITACC
   // Debugging build (-DLD2_WAITACC), used with lab200_la_debug_trace: lane 0 of every warp of CTA (0, 0, 0) sums the cycles it
   // spends inside bounded waits, per barrier, and the clock at a few events per block, and writes the sums behind the per-block
-  // stamps: trace[blocks * LA_TRACE_SLOTS + 16 + warp * LD2_NUM_BARS + barrier] and, after those 15 rows, [warp * 8 + event].
+  // stamps: trace[blocks * LA_TRACE_SLOTS + 16 + warp * LD2_NUM_BARS + barrier] and, after those 16 rows, [warp * 8 + event].
   // The trace buffer must have room for them. Dividing by the block count gives the average wait per block and, relative to
   // the MMA warp's event 0, the average time of each event inside a block.
   long long wait_acc = 0;
@@ -172,184 +176,188 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #define LD2_TRACE(slot, it) LD2_STAMP(slot, it)
 #define LD2_WAIT(which, it, code) if (!lap_wait(bar(which, it), par(it), abort_flag, budget)) { LD2_FAIL(code) break; }
 
-  if (warp == 0) {
-    // =========================================== TMA loads ==============================================
-    // Prologue: everything block 0 needs, do of block 1, and (once Vs of block 0 exists) v of block 1. Then, per block it,
-    // the reloads in the order in which their buffers come free: q (D has read it), k (Ks exists), do two blocks ahead
-    // (P1 do has read the stage), v two blocks ahead (Vs of the next block exists).
-    if (issuer_lane(lane)) {
-      auto load_q = [&](int i) {
-        mbar_arrive_expect_tx(bar(LD2_FULL_Q, i), 2 * SLAB);
-        for (int sl = 0; sl < 2; ++sl)  // q always as two slabs: it is the M = 128 side of the state MMA
-          tma_load_3d(sQ + sl * SLAB, &tmQ, sl * 64, blk_of(i) * LA_BLOCK, zc, bar(LD2_FULL_Q, i));
-      };
-      auto load_k = [&](int i) {
-        mbar_arrive_expect_tx(bar(LD2_FULL_K, i), ND * SLAB);
-        for (int sl = 0; sl < ND; ++sl) tma_load_3d(sK + sl * SLAB, &tmK, sl * 64, blk_of(i) * LA_BLOCK, zc, bar(LD2_FULL_K, i));
-      };
-      auto load_v = [&](int i) {
-        mbar_arrive_expect_tx(bar(LD2_FULL_V, i), NE * SLAB);
-        for (int sl = 0; sl < NE; ++sl) tma_load_3d(sV + sl * SLAB, &tmV, sl * 64, blk_of(i) * LA_BLOCK, zc, bar(LD2_FULL_V, i));
-      };
-      auto load_g = [&](int i) {
-        mbar_arrive_expect_tx(bar(LD2_FULL_G, i), NE * SLAB);
-        for (int sl = 0; sl < NE; ++sl)
-          tma_load_3d(sG + ((i & 1) * 2 + sl) * SLAB, &tmG, sl * 64, blk_of(i) * LA_BLOCK, zc, bar(LD2_FULL_G, i));
-      };
-      if (nb > 0) {
-        load_v(0); load_g(0); load_k(0); load_q(0);
-        if (nb > 1) load_g(1);
-      }
-      do {
-        if (nb > 1) {
-          LD2_WAIT(LD2_PV0_READY, 0, LA_ERR_WAIT_MMA1)
-          load_v(1);
+  if (warp < 4) {
+    regs_set<128, LD2_REGS[0]>();
+    if (warp == 0) {
+      // =========================================== TMA loads ==============================================
+      // Prologue: everything block 0 needs, do of block 1, and (once Vs of block 0 exists) v of block 1. Then, per block it,
+      // the reloads in the order in which their buffers come free: q (D has read it), k (Ks exists), do two blocks ahead
+      // (P1 do has read the stage), v two blocks ahead (Vs of the next block exists).
+      if (issuer_lane(lane)) {
+        auto load_q = [&](int i) {
+          mbar_arrive_expect_tx(bar(LD2_FULL_Q, i), 2 * SLAB);
+          for (int sl = 0; sl < 2; ++sl)  // q always as two slabs: it is the M = 128 side of the state MMA
+            tma_load_3d(sQ + sl * SLAB, &tmQ, sl * 64, blk_of(i) * LA_BLOCK, zc, bar(LD2_FULL_Q, i));
+        };
+        auto load_k = [&](int i) {
+          mbar_arrive_expect_tx(bar(LD2_FULL_K, i), ND * SLAB);
+          for (int sl = 0; sl < ND; ++sl) tma_load_3d(sK + sl * SLAB, &tmK, sl * 64, blk_of(i) * LA_BLOCK, zc, bar(LD2_FULL_K, i));
+        };
+        auto load_v = [&](int i) {
+          mbar_arrive_expect_tx(bar(LD2_FULL_V, i), NE * SLAB);
+          for (int sl = 0; sl < NE; ++sl) tma_load_3d(sV + sl * SLAB, &tmV, sl * 64, blk_of(i) * LA_BLOCK, zc, bar(LD2_FULL_V, i));
+        };
+        auto load_g = [&](int i) {
+          mbar_arrive_expect_tx(bar(LD2_FULL_G, i), NE * SLAB);
+          for (int sl = 0; sl < NE; ++sl)
+            tma_load_3d(sG + ((i & 1) * 2 + sl) * SLAB, &tmG, sl * 64, blk_of(i) * LA_BLOCK, zc, bar(LD2_FULL_G, i));
+        };
+        if (nb > 0) {
+          load_v(0); load_g(0); load_k(0); load_q(0);
+          if (nb > 1) load_g(1);
         }
+        do {
+          if (nb > 1) {
+            LD2_WAIT(LD2_PV0_READY, 0, LA_ERR_WAIT_MMA1)
+            load_v(1);
+          }
+          for (int it = 0; it < nb; ++it) {
+            if (it + 1 < nb) {
+              // q and k of the next block go to L2 now, a block before their loads: those loads sit in the chains that bound
+              // the block (D -> q -> S1, Ks -> k -> S1) and complete in ~1,300 cycles from L2 instead of ~2,800 from HBM.
+              // (Prefetching v and do as well was measured slower.)
+              for (int sl = 0; sl < 2; ++sl) tma_prefetch_l2_3d(&tmQ, sl * 64, blk_of(it + 1) * LA_BLOCK, zc);
+              for (int sl = 0; sl < ND; ++sl) tma_prefetch_l2_3d(&tmK, sl * 64, blk_of(it + 1) * LA_BLOCK, zc);
+            }
+            if (it + 1 < nb) {
+              LD2_WAIT(LD2_D_DONE, it, LA_ERR_WAIT_MMA2)
+              load_q(it + 1);
+              LD2_EV(0)
+              LD2_WAIT(LD2_PK1_READY, it, LA_ERR_WAIT_MMA1)
+              load_k(it + 1);
+              LD2_EV(1)
+            }
+            if (it + 2 < nb) {
+              LD2_WAIT(LD2_PC1_DONE, it, LA_ERR_WAIT_MMA2)
+              load_g(it + 2);
+              LD2_EV(2)
+              LD2_WAIT(LD2_PV0_READY, it + 1, LA_ERR_WAIT_MMA1)
+              load_v(it + 2);
+              LD2_EV(3)
+            }
+          }
+        } while (false);
+      }
+    } else if (warp == 2) {
+      // =========================================== TMA stores =============================================
+      // The two staged output tiles of a block leave in turn through the one staging buffer.
+      if (issuer_lane(lane)) {
         for (int it = 0; it < nb; ++it) {
-          if (it + 1 < nb) {
-            // q and k of the next block go to L2 now, a block before their loads: those loads sit in the chains that bound
-            // the block (D -> q -> S1, Ks -> k -> S1) and complete in ~1,300 cycles from L2 instead of ~2,800 from HBM.
-            // (Prefetching v and do as well was measured slower.)
-            for (int sl = 0; sl < 2; ++sl) tma_prefetch_l2_3d(&tmQ, sl * 64, blk_of(it + 1) * LA_BLOCK, zc);
-            for (int sl = 0; sl < ND; ++sl) tma_prefetch_l2_3d(&tmK, sl * 64, blk_of(it + 1) * LA_BLOCK, zc);
-          }
-          if (it + 1 < nb) {
-            LD2_WAIT(LD2_D_DONE, it, LA_ERR_WAIT_MMA2)
-            load_q(it + 1);
-            LD2_EV(0)
-            LD2_WAIT(LD2_PK1_READY, it, LA_ERR_WAIT_MMA1)
-            load_k(it + 1);
-            LD2_EV(1)
-          }
-          if (it + 2 < nb) {
-            LD2_WAIT(LD2_PC1_DONE, it, LA_ERR_WAIT_MMA2)
-            load_g(it + 2);
-            LD2_EV(2)
-            LD2_WAIT(LD2_PV0_READY, it + 1, LA_ERR_WAIT_MMA1)
-            load_v(it + 2);
-            LD2_EV(3)
-          }
-        }
-      } while (false);
-    }
-  } else if (warp == 14) {
-    // =========================================== TMA stores =============================================
-    // The two staged output tiles of a block leave in turn through the one staging buffer.
-    if (issuer_lane(lane)) {
-      for (int it = 0; it < nb; ++it) {
-        bool ok = true;
+          bool ok = true;
 #pragma unroll 1
-        for (int u = 0; u < 2 && ok; ++u) {
-          ok = lap_wait(bar(u ? LD2_O_STAGED1 : LD2_O_STAGED0, it), par(it), abort_flag, budget);
-          if (!ok) break;
-          const int nslab = u ? NE : ND;
-          for (int sl = 0; sl < nslab; ++sl)
-            tma_store_3d(u ? static_cast<const void*>(&tmDV) : static_cast<const void*>(&tmDK), sO + sl * SLAB, sl * 64,
-                         blk_of(it) * LA_BLOCK, zc);
-          tma_store_commit();
-          tma_store_wait_read();
-          mbar_arrive(bar(u ? LD2_BUF_FREE1 : LD2_BUF_FREE0, it));
-          LD2_EV(u)
-        }
-        if (!ok) { LD2_FAIL(LA_ERR_WAIT_MMA2) break; }
-      }
-      tma_store_wait_all();
-    }
-  } else if (warp == 1) {
-    // ============================================ MMA issuer ============================================
-    if (issuer_lane(lane)) {
-      auto issue_S0 = [&](int i) -> bool {  // S0 = v do^T (contraction over e)
-        if (!lap_wait(bar(LD2_FULL_V, i), par(i), abort_flag, budget)) return false;
-        if (!lap_wait(bar(LD2_FULL_G, i), par(i), abort_flag, budget)) return false;
-        tc_fence_after_sync();
-        const uint32_t g0 = sG + (i & 1) * 2 * SLAB;
-        for (int kq = 0; kq < ne16; ++kq) {
-          const uint32_t off = (kq >> 2) * SLAB + (kq & 3) * 32;
-          umma_f16(tmem + T_SA, smem_desc_sw128(sV + off, 16), smem_desc_sw128(g0 + off, 16), IDESC_S, kq > 0);
-        }
-        umma_commit(bar(LD2_S0_READY, i));
-        return true;
-      };
-      auto issue_S1 = [&](int i) -> bool {  // S1 = k q^T (contraction over d)
-        if (!lap_wait(bar(LD2_FULL_K, i), par(i), abort_flag, budget)) return false;
-        if (!lap_wait(bar(LD2_FULL_Q, i), par(i), abort_flag, budget)) return false;
-        tc_fence_after_sync();
-        for (int kq = 0; kq < nd16; ++kq) {
-          const uint32_t off = (kq >> 2) * SLAB + (kq & 3) * 32;
-          umma_f16(tmem + T_SB, smem_desc_sw128(sK + off, 16), smem_desc_sw128(sQ + off, 16), IDESC_S, kq > 0);
-        }
-        umma_commit(bar(LD2_S1_READY, i));
-        return true;
-      };
-      bool alive = true;
-      if (nb > 0) {
-        alive = issue_S0(0) && issue_S1(0);
-        if (!alive) LD2_FAIL(LA_ERR_WAIT_INPUT)
-      }
-      for (int it = 0; it < nb && alive; ++it) {
-        const uint32_t sGs = sG + (it & 1) * 2 * SLAB;
-        const bool have_state = have_state_in || (it > 0);
-        LD2_TRACE(0, it)
-        LD2_EV(0)
-        // ---- dk = P0 q + Vs dKV^T; the first half is the last reader of the unscaled q tile ----------------------------
-        LD2_WAIT(LD2_PV0_READY, it, LA_ERR_WAIT_MMA1)
-        if (it > 0) { LD2_WAIT(LD2_O_FREE1, it - 1, LA_ERR_WAIT_MMA2) }  // the dv epilogue of the previous block has read O
-        tc_fence_after_sync();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_f16_ts(tmem + T_O, tmem + T_SA + kk * 8, smem_desc_sw128(sQ + kk * 2048, SLAB), IDESC_PC0, kk > 0);
-        umma_commit(bar(LD2_QP_DONE, it));
-        LD2_TRACE(1, it)
-        LD2_EV(1)
-        if (have_state) {
-          LD2_WAIT(LD2_STATE_READY, it, LA_ERR_WAIT_MMA2)
-          tc_fence_after_sync();
-          for (int kq = 0; kq < ne16; ++kq) {  // contraction over e: state copy columns
-            const uint32_t off = (kq >> 2) * SLAB + (kq & 3) * 32;
-            umma_f16_ts(tmem + T_O, tmem + T_SA + T_XA + kq * 8, smem_desc_sw128(sS + off, 16), IDESC_X0, 1);
+          for (int u = 0; u < 2 && ok; ++u) {
+            ok = lap_wait(bar(u ? LD2_O_STAGED1 : LD2_O_STAGED0, it), par(it), abort_flag, budget);
+            if (!ok) break;
+            const int nslab = u ? NE : ND;
+            for (int sl = 0; sl < nslab; ++sl)
+              tma_store_3d(u ? static_cast<const void*>(&tmDV) : static_cast<const void*>(&tmDK), sO + sl * SLAB, sl * 64,
+                           blk_of(it) * LA_BLOCK, zc);
+            tma_store_commit();
+            tma_store_wait_read();
+            mbar_arrive(bar(u ? LD2_BUF_FREE1 : LD2_BUF_FREE0, it));
+            LD2_EV(u)
           }
+          if (!ok) { LD2_FAIL(LA_ERR_WAIT_MMA2) break; }
         }
-        umma_commit(bar(LD2_PC0_DONE, it));
-        LD2_TRACE(2, it)
-        LD2_EV(2)
-        if (it + 1 < nb) {
-          if (!issue_S0(it + 1)) { LD2_FAIL(LA_ERR_WAIT_INPUT) break; }
+        tma_store_wait_all();
+      }
+    } else if (warp == 1) {
+      // ============================================ MMA issuer ============================================
+      if (issuer_lane(lane)) {
+        auto issue_S0 = [&](int i) -> bool {  // S0 = v do^T (contraction over e)
+          if (!lap_wait(bar(LD2_FULL_V, i), par(i), abort_flag, budget)) return false;
+          if (!lap_wait(bar(LD2_FULL_G, i), par(i), abort_flag, budget)) return false;
+          tc_fence_after_sync();
+          const uint32_t g0 = sG + (i & 1) * 2 * SLAB;
+          for (int kq = 0; kq < ne16; ++kq) {
+            const uint32_t off = (kq >> 2) * SLAB + (kq & 3) * 32;
+            umma_f16(tmem + T_SA, smem_desc_sw128(sV + off, 16), smem_desc_sw128(g0 + off, 16), IDESC_S, kq > 0);
+          }
+          umma_commit(bar(LD2_S0_READY, i));
+          return true;
+        };
+        auto issue_S1 = [&](int i) -> bool {  // S1 = k q^T (contraction over d)
+          if (!lap_wait(bar(LD2_FULL_K, i), par(i), abort_flag, budget)) return false;
+          if (!lap_wait(bar(LD2_FULL_Q, i), par(i), abort_flag, budget)) return false;
+          tc_fence_after_sync();
+          for (int kq = 0; kq < nd16; ++kq) {
+            const uint32_t off = (kq >> 2) * SLAB + (kq & 3) * 32;
+            umma_f16(tmem + T_SB, smem_desc_sw128(sK + off, 16), smem_desc_sw128(sQ + off, 16), IDESC_S, kq > 0);
+          }
+          umma_commit(bar(LD2_S1_READY, i));
+          return true;
+        };
+        bool alive = true;
+        if (nb > 0) {
+          alive = issue_S0(0) && issue_S1(0);
+          if (!alive) LD2_FAIL(LA_ERR_WAIT_INPUT)
         }
-        LD2_TRACE(3, it)
-        LD2_EV(3)
-        // ---- D = (w_state q)^T do: the last reader of q ------------------------------------------------------------------
-        LD2_WAIT(LD2_Q_SCALED, it, LA_ERR_WAIT_MMA2)
-        if (it > 0) { LD2_WAIT(LD2_D_FREE, it - 1, LA_ERR_WAIT_MMA2) }
-        tc_fence_after_sync();
+        for (int it = 0; it < nb && alive; ++it) {
+          const uint32_t sGs = sG + (it & 1) * 2 * SLAB;
+          const bool have_state = have_state_in || (it > 0);
+          LD2_TRACE(0, it)
+          LD2_EV(0)
+          // ---- dk = P0 q + Vs dKV^T; the first half is the last reader of the unscaled q tile ----------------------------
+          LD2_WAIT(LD2_PV0_READY, it, LA_ERR_WAIT_MMA1)
+          if (it > 0) { LD2_WAIT(LD2_O_FREE1, it - 1, LA_ERR_WAIT_MMA2) }  // the dv epilogue of the previous block has read O
+          tc_fence_after_sync();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_f16(tmem + T_D, smem_desc_sw128(sQ + kk * 2048, SLAB), smem_desc_sw128(sGs + kk * 2048, SLAB), IDESC_D, kk > 0);
-        umma_commit(bar(LD2_D_DONE, it));
-        LD2_TRACE(7, it)
-        LD2_EV(4)
-        // ---- dv = P1 do + Ks dKV -----------------------------------------------------------------------------------
-        LD2_WAIT(LD2_PK1_READY, it, LA_ERR_WAIT_MMA1)
-        LD2_WAIT(LD2_O_FREE0, it, LA_ERR_WAIT_MMA2)  // the dk epilogue has read O
-        LD2_TRACE(4, it)
-        tc_fence_after_sync();
+          for (int kk = 0; kk < 8; ++kk)
+            umma_f16_ts(tmem + T_O, tmem + T_SA + kk * 8, smem_desc_sw128(sQ + kk * 2048, SLAB), IDESC_PC0, kk > 0);
+          umma_commit(bar(LD2_QP_DONE, it));
+          LD2_TRACE(1, it)
+          LD2_EV(1)
+          if (have_state) {
+            LD2_WAIT(LD2_STATE_READY, it, LA_ERR_WAIT_MMA2)
+            tc_fence_after_sync();
+            for (int kq = 0; kq < ne16; ++kq) {  // contraction over e: state copy columns
+              const uint32_t off = (kq >> 2) * SLAB + (kq & 3) * 32;
+              umma_f16_ts(tmem + T_O, tmem + T_SA + T_XA + kq * 8, smem_desc_sw128(sS + off, 16), IDESC_X0, 1);
+            }
+          }
+          umma_commit(bar(LD2_PC0_DONE, it));
+          LD2_TRACE(2, it)
+          LD2_EV(2)
+          if (it + 1 < nb) {
+            if (!issue_S0(it + 1)) { LD2_FAIL(LA_ERR_WAIT_INPUT) break; }
+          }
+          LD2_TRACE(3, it)
+          LD2_EV(3)
+          // ---- D = (w_state q)^T do: the last reader of q ------------------------------------------------------------------
+          LD2_WAIT(LD2_Q_SCALED, it, LA_ERR_WAIT_MMA2)
+          if (it > 0) { LD2_WAIT(LD2_D_FREE, it - 1, LA_ERR_WAIT_MMA2) }
+          tc_fence_after_sync();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_f16_ts(tmem + T_O, tmem + T_SB + kk * 8, smem_desc_sw128(sGs + kk * 2048, SLAB), IDESC_PC1, kk > 0);
-        if (have_state) {
-          for (int kq = 0; kq < nd16; ++kq)  // contraction over d: state copy rows
-            umma_f16_ts(tmem + T_O, tmem + T_SB + T_XA + kq * 8, smem_desc_sw128(sS + kq * 2048, SLAB), IDESC_X1, 1);
+          for (int kk = 0; kk < 8; ++kk)
+            umma_f16(tmem + T_D, smem_desc_sw128(sQ + kk * 2048, SLAB), smem_desc_sw128(sGs + kk * 2048, SLAB), IDESC_D, kk > 0);
+          umma_commit(bar(LD2_D_DONE, it));
+          LD2_TRACE(7, it)
+          LD2_EV(4)
+          // ---- dv = P1 do + Ks dKV -----------------------------------------------------------------------------------
+          LD2_WAIT(LD2_PK1_READY, it, LA_ERR_WAIT_MMA1)
+          LD2_WAIT(LD2_O_FREE0, it, LA_ERR_WAIT_MMA2)  // the dk epilogue has read O
+          LD2_TRACE(4, it)
+          tc_fence_after_sync();
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            umma_f16_ts(tmem + T_O, tmem + T_SB + kk * 8, smem_desc_sw128(sGs + kk * 2048, SLAB), IDESC_PC1, kk > 0);
+          if (have_state) {
+            for (int kq = 0; kq < nd16; ++kq)  // contraction over d: state copy rows
+              umma_f16_ts(tmem + T_O, tmem + T_SB + T_XA + kq * 8, smem_desc_sw128(sS + kq * 2048, SLAB), IDESC_X1, 1);
+          }
+          umma_commit(bar(LD2_PC1_DONE, it));
+          LD2_TRACE(5, it)
+          LD2_EV(5)
+          if (it + 1 < nb) {
+            if (!issue_S1(it + 1)) { LD2_FAIL(LA_ERR_WAIT_INPUT) break; }
+          }
+          LD2_TRACE(6, it)
+          LD2_EV(6)
         }
-        umma_commit(bar(LD2_PC1_DONE, it));
-        LD2_TRACE(5, it)
-        LD2_EV(5)
-        if (it + 1 < nb) {
-          if (!issue_S1(it + 1)) { LD2_FAIL(LA_ERR_WAIT_INPUT) break; }
-        }
-        LD2_TRACE(6, it)
-        LD2_EV(6)
       }
     }
-  } else if (warp < 6) {
+  } else if (warp < 8) {
+    regs_set<128, LD2_REGS[1]>();
     // ============================================ mask group ============================================
     // Reverse-time mask on both products: keep c >= r with lambda^(c-r). One warp per TMEM lane quadrant, four 32-column
     // tiles each, in column order; P tile t goes back over S columns [16 t, 16 t + 16), which the warp has read by then.
@@ -450,7 +458,8 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else {
     // ========================================= state / output group =====================================
-    const int w8 = warp - 6;
+    regs_set<128, LD2_REGS[2]>();
+    const int w8 = warp - 8;
     const int q = warp & 3, hf = w8 >> 2;
     const int r = q * 32 + lane;
     const uint32_t lanebase = static_cast<uint32_t>(q * 32) << 16;
@@ -604,7 +613,7 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (p.trace != nullptr && bh == 0 && blockIdx.y == 0 && lane == 0)
     for (int i = 0; i < LD2_NUM_BARS; ++i) p.trace[p.trace_blocks * LA_TRACE_SLOTS + 16 + warp * LD2_NUM_BARS + i] = wait_site[i];
   if (p.trace != nullptr && bh == 0 && blockIdx.y == 0 && lane == 0)
-    for (int i = 0; i < 8; ++i) p.trace[p.trace_blocks * LA_TRACE_SLOTS + 16 + 15 * LD2_NUM_BARS + warp * 8 + i] = ev_sum[i];
+    for (int i = 0; i < 8; ++i) p.trace[p.trace_blocks * LA_TRACE_SLOTS + 16 + 16 * LD2_NUM_BARS + warp * 8 + i] = ev_sum[i];
 #undef LD2_EV
 #endif
 #undef LD2_WAIT

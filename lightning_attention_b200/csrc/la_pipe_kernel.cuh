@@ -4,8 +4,8 @@
 //
 //   warp 0      TMA producer   loads A, Bm, C tiles of block i+1, i+2 into two shared-memory stages
 //   warp 1      MMA issuer     X_i = A State_i, D_i = C^T (w Bm), PC_i = P_i C, S_{i+1} = A Bm^T, in this order (one thread)
-//   warps 2-5   mask group     S_i (TMEM) -> decay mask -> P_i (bf16, back into TMEM over S)
-//   warps 6-13  state/output   Bm_i rows *= w_state (for D_i); D_i -> StateT = lambda^128 StateT + D_i (fp32 registers)
+//   warps 4-7   mask group     S_i (TMEM) -> decay mask -> P_i (bf16, back into TMEM over S)
+//   warps 8-15  state/output   Bm_i rows *= w_state (for D_i); D_i -> StateT = lambda^128 StateT + D_i (fp32 registers)
 //                              -> bf16 copy for X_{i+1}; O_i = PC_i + w_out X_i -> swizzled shared-memory tile -> TMA store
 //
 // P never touches shared memory: it is written to TMEM with tcgen05.st and consumed by tcgen05.mma as the
@@ -25,7 +25,13 @@
 
 namespace lab200 {
 
-constexpr int LAP_THREADS = 448;
+// Four warpgroups: loads and MMAs (two of its warps idle), mask, and two of the state/output group. The launch gives every thread
+// 128 registers; the fp32 state and the tiles beside it need more, the issuing threads far less, so the warpgroups split what
+// the launch was given. At 128 for all, the loops spilled 124-144 bytes per thread, and what spills goes through the shared-memory
+// pipe that bounds the kernel: b4 h32 n2048 d=e=128 forward 53.4 -> 51.4 us, n32768 forward 851 -> 823.
+constexpr int LAP_THREADS = 512;
+constexpr int LAP_REGS[3] = {56, 120, 168};
+static_assert(LAP_REGS[0] + LAP_REGS[1] + 2 * LAP_REGS[2] <= 512, "the split must not ask for more than the launch gave");
 constexpr int LAP_MASK_THREADS = 128, LAP_STATE_THREADS = 256;
 
 
@@ -166,153 +172,157 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #define LAP_TRACE(slot, it) if (p.trace != nullptr && bh == 0 && blockIdx.x == 0 && blockIdx.y == 0 && (it) < p.trace_blocks) \
     p.trace[(it) * LA_TRACE_SLOTS + (slot)] = clock64();
 
-  if (warp == 0) {
-    // =========================================== TMA producer ===========================================
-    // Also issues the TMA stores of the output tiles: a tile is staged in the C stage of its block (P C, the last MMA of a
-    // block, has read C by then), and that stage is reloaded (for block it+2) only after the store has read it.
-    if (issuer_lane(lane)) {
-      auto blk_of = [&](int i) { return reverse ? (blk_end - 1 - i) : (blk_begin + i); };
-      auto store_tile = [&](int i) -> bool {  // output tile of block i: wait until it is staged, then store it
-        const int sst = i & 1;
-        if (!lap_wait(bar(LAP_O_STAGED, sst), (i >> 1) & 1, abort_flag, budget)) return false;
+  if (warp < 4) {
+    regs_set<128, LAP_REGS[0]>();
+    if (warp == 0) {
+      // =========================================== TMA producer ===========================================
+      // Also issues the TMA stores of the output tiles: a tile is staged in the C stage of its block (P C, the last MMA of a
+      // block, has read C by then), and that stage is reloaded (for block it+2) only after the store has read it.
+      if (issuer_lane(lane)) {
+        auto blk_of = [&](int i) { return reverse ? (blk_end - 1 - i) : (blk_begin + i); };
+        auto store_tile = [&](int i) -> bool {  // output tile of block i: wait until it is staged, then store it
+          const int sst = i & 1;
+          if (!lap_wait(bar(LAP_O_STAGED, sst), (i >> 1) & 1, abort_flag, budget)) return false;
 #pragma unroll
-        for (int vs = 0; vs < NVS; ++vs)
-          tma_store_3d(&tmO, sC + (sst * NCS + vs) * SLAB, dv_off + vs * 64, blk_of(i) * LA_BLOCK, zc);
-        tma_store_commit();
-        return true;
-      };
-      bool alive = true;
-      for (int it = 0; it < nb && alive; ++it) {
-        const int blk = blk_of(it);
-        const int st = it & 1;
-        const uint32_t prev_par = ((it >> 1) & 1) ^ 1;  // parity of the previous use of this stage (block it-2)
-        // A and Bm of block it: their stages are free once every MMA of block it-2 has run (P C is the last one issued; in
-        // state-only mode D). They are what S of block it waits for, so they go first and wait for nothing else.
-        // Where there is one stage, A is free after X of block it-1 and Bm after D of block it-1.
-        const uint32_t last_par = ((it - 1) >> 1) & 1;
-        auto load_b = [&]() {
-#pragma unroll
-          for (int ks = 0; ks < NKS; ++ks)
-            tma_load_3d(sB + (st * NBS + ks) * SLAB, &tmB, ks * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_AB, st));
+          for (int vs = 0; vs < NVS; ++vs)
+            tma_store_3d(&tmO, sC + (sst * NCS + vs) * SLAB, dv_off + vs * 64, blk_of(i) * LA_BLOCK, zc);
+          tma_store_commit();
+          return true;
         };
-        if (NBS != 0 && it >= 2) {
-          if (!lap_wait(bar(MODE == 0 ? LAP_PC_DONE : LAP_D_DONE, st), prev_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
-        }
-        mbar_arrive_expect_tx(bar(LAP_FULL_AB, st), (MODE == 0 ? 2 * NKS : NKS) * SLAB);
-        if (NBS != 0) load_b();
-        if (MODE == 0) {
-          if (NAS == 0 && it >= 1 && !lap_wait(bar(LAP_A_FREE, st ^ 1), last_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+        bool alive = true;
+        for (int it = 0; it < nb && alive; ++it) {
+          const int blk = blk_of(it);
+          const int st = it & 1;
+          const uint32_t prev_par = ((it >> 1) & 1) ^ 1;  // parity of the previous use of this stage (block it-2)
+          // A and Bm of block it: their stages are free once every MMA of block it-2 has run (P C is the last one issued; in
+          // state-only mode D). They are what S of block it waits for, so they go first and wait for nothing else.
+          // Where there is one stage, A is free after X of block it-1 and Bm after D of block it-1.
+          const uint32_t last_par = ((it - 1) >> 1) & 1;
+          auto load_b = [&]() {
 #pragma unroll
-          for (int ks = 0; ks < NKS; ++ks)
-            tma_load_3d(sA + (st * NAS + ks) * SLAB, &tmA, ks * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_AB, st));
-        }
-        if (NBS == 0) {
-          if (it >= 1 && !lap_wait(bar(LAP_D_DONE, st ^ 1), last_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
-          load_b();
-        }
-        // C of block it: in the full block loop its stage holds the staged output tile of block it-2, which is stored first;
-        // C is not needed before D of block it, a whole block later than A and Bm.
-        if (MODE == 0 && it >= 2) {
-          if (!store_tile(it - 2)) { LAP_FAIL(LA_ERR_WAIT_MMA2) alive = false; break; }
-          tma_store_wait_read();
-        }
-        // Only the slabs of this CTA's dv slice are loaded. D = C^T (w Bm) is an M = 128 MMA and reads both slabs of the stage; with
-        // a 64-wide slice the second one holds stale bytes, which only reach accumulator rows >= 64 that nobody reads.
-        mbar_arrive_expect_tx(bar(LAP_FULL_C, st), NVS * SLAB);
+            for (int ks = 0; ks < NKS; ++ks)
+              tma_load_3d(sB + (st * NBS + ks) * SLAB, &tmB, ks * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_AB, st));
+          };
+          if (NBS != 0 && it >= 2) {
+            if (!lap_wait(bar(MODE == 0 ? LAP_PC_DONE : LAP_D_DONE, st), prev_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+          }
+          mbar_arrive_expect_tx(bar(LAP_FULL_AB, st), (MODE == 0 ? 2 * NKS : NKS) * SLAB);
+          if (NBS != 0) load_b();
+          if (MODE == 0) {
+            if (NAS == 0 && it >= 1 && !lap_wait(bar(LAP_A_FREE, st ^ 1), last_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
 #pragma unroll
-        for (int vs = 0; vs < NVS; ++vs)
-          tma_load_3d(sC + (st * NCS + vs) * SLAB, &tmC, dv_off + vs * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_C, st));
-      }
-      if (MODE == 0 && alive && *abort_flag == 0) {
-        for (int i = max(nb - 2, 0); i < nb; ++i) {
-          if (!store_tile(i)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+            for (int ks = 0; ks < NKS; ++ks)
+              tma_load_3d(sA + (st * NAS + ks) * SLAB, &tmA, ks * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_AB, st));
+          }
+          if (NBS == 0) {
+            if (it >= 1 && !lap_wait(bar(LAP_D_DONE, st ^ 1), last_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+            load_b();
+          }
+          // C of block it: in the full block loop its stage holds the staged output tile of block it-2, which is stored first;
+          // C is not needed before D of block it, a whole block later than A and Bm.
+          if (MODE == 0 && it >= 2) {
+            if (!store_tile(it - 2)) { LAP_FAIL(LA_ERR_WAIT_MMA2) alive = false; break; }
+            tma_store_wait_read();
+          }
+          // Only the slabs of this CTA's dv slice are loaded. D = C^T (w Bm) is an M = 128 MMA and reads both slabs of the stage; with
+          // a 64-wide slice the second one holds stale bytes, which only reach accumulator rows >= 64 that nobody reads.
+          mbar_arrive_expect_tx(bar(LAP_FULL_C, st), NVS * SLAB);
+#pragma unroll
+          for (int vs = 0; vs < NVS; ++vs)
+            tma_load_3d(sC + (st * NCS + vs) * SLAB, &tmC, dv_off + vs * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_C, st));
         }
-      }
-      if (MODE == 0) tma_store_wait_all();
-    }
-  } else if (warp == 1) {
-    // ============================================ MMA issuer ============================================
-    // Issue order per block: X_i, D_i, PC_i, S_{i+1}. X_i and D_i need nothing from the mask group, so they run while
-    // it turns S_i into P_i; D_i this early also means the next state is ready long before X_{i+1} asks for it.
-    // S_{i+1} overwrites the TMEM columns P_i lives in, so it follows PC_i (the tensor pipe executes in issue order).
-    // D and P C commit to their own barriers: the state update starts after D_i, the output tile leaves TMEM after
-    // PC_i while S_{i+1}, X_{i+1} and D_{i+1} run.
-    if (issuer_lane(lane)) {
-      auto issue_S = [&](int i) -> bool {
-        const int ist = i & 1;
-        if (!lap_wait(bar(LAP_FULL_AB, ist), (i >> 1) & 1, abort_flag, budget)) return false;
-        tc_fence_after_sync();
-        const uint32_t a0 = sA + ist * NAS * SLAB, b0 = sB + ist * NBS * SLAB;
-        for (int kq = 0; kq < nk16; ++kq) {  // S = A Bm^T
-          const uint32_t off = (kq >> 2) * SLAB + (kq & 3) * 32;
-          umma_f16(tmem + T_S, smem_desc_sw128(a0 + off, 16), smem_desc_sw128(b0 + off, 16), IDESC_S, kq > 0);
+        if (MODE == 0 && alive && *abort_flag == 0) {
+          for (int i = max(nb - 2, 0); i < nb; ++i) {
+            if (!store_tile(i)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+          }
         }
-        umma_commit(bar(LAP_S_READY, ist));
-        return true;
-      };
-      bool alive = true;
-      if (MODE == 0 && nb > 0) {
-        alive = issue_S(0);
-        if (!alive) LAP_FAIL(LA_ERR_WAIT_INPUT)
+        if (MODE == 0) tma_store_wait_all();
       }
-      for (int it = 0; it < nb && alive; ++it) {
-        const int st = it & 1;
-        const uint32_t par = (it >> 1) & 1;
-        const int pst = st ^ 1;                         // instance used by block it-1
-        const uint32_t ppar = ((it - 1) >> 1) & 1;      // and its parity
-        const uint32_t sAs = sA + st * NAS * SLAB, sBs = sB + st * NBS * SLAB, sCs = sC + st * NCS * SLAB;
-        const bool have_state = have_state_in || (it > 0);
-        LAP_TRACE(0, it)
-        if (MODE == 0) {
-          if (have_state) {
-            if (!lap_wait(bar(LAP_STATE_READY, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
-            if (it > 0 && !lap_wait(bar(LAP_O_FREE, pst), ppar, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
-            tc_fence_after_sync();
-            for (int kq = 0; kq < nk16; ++kq) {  // X = A State
-              const uint32_t offA = (kq >> 2) * SLAB + (kq & 3) * 32;
-              if constexpr (WIDE) {
-                umma_f16(tmem + T_OX, smem_desc_sw128(sAs + offA, 16), smem_desc_sw128(sS + kq * 2048, SLAB), IDESC_PC, kq > 0);
-              } else {
-                const uint32_t offS = (kq >> 2) * (DV * 128) + (kq & 3) * 32;
-                umma_f16(tmem + T_OX, smem_desc_sw128(sAs + offA, 16), smem_desc_sw128(sS + offS, 16), IDESC_X, kq > 0);
+    } else if (warp == 1) {
+      // ============================================ MMA issuer ============================================
+      // Issue order per block: X_i, D_i, PC_i, S_{i+1}. X_i and D_i need nothing from the mask group, so they run while
+      // it turns S_i into P_i; D_i this early also means the next state is ready long before X_{i+1} asks for it.
+      // S_{i+1} overwrites the TMEM columns P_i lives in, so it follows PC_i (the tensor pipe executes in issue order).
+      // D and P C commit to their own barriers: the state update starts after D_i, the output tile leaves TMEM after
+      // PC_i while S_{i+1}, X_{i+1} and D_{i+1} run.
+      if (issuer_lane(lane)) {
+        auto issue_S = [&](int i) -> bool {
+          const int ist = i & 1;
+          if (!lap_wait(bar(LAP_FULL_AB, ist), (i >> 1) & 1, abort_flag, budget)) return false;
+          tc_fence_after_sync();
+          const uint32_t a0 = sA + ist * NAS * SLAB, b0 = sB + ist * NBS * SLAB;
+          for (int kq = 0; kq < nk16; ++kq) {  // S = A Bm^T
+            const uint32_t off = (kq >> 2) * SLAB + (kq & 3) * 32;
+            umma_f16(tmem + T_S, smem_desc_sw128(a0 + off, 16), smem_desc_sw128(b0 + off, 16), IDESC_S, kq > 0);
+          }
+          umma_commit(bar(LAP_S_READY, ist));
+          return true;
+        };
+        bool alive = true;
+        if (MODE == 0 && nb > 0) {
+          alive = issue_S(0);
+          if (!alive) LAP_FAIL(LA_ERR_WAIT_INPUT)
+        }
+        for (int it = 0; it < nb && alive; ++it) {
+          const int st = it & 1;
+          const uint32_t par = (it >> 1) & 1;
+          const int pst = st ^ 1;                         // instance used by block it-1
+          const uint32_t ppar = ((it - 1) >> 1) & 1;      // and its parity
+          const uint32_t sAs = sA + st * NAS * SLAB, sBs = sB + st * NBS * SLAB, sCs = sC + st * NCS * SLAB;
+          const bool have_state = have_state_in || (it > 0);
+          LAP_TRACE(0, it)
+          if (MODE == 0) {
+            if (have_state) {
+              if (!lap_wait(bar(LAP_STATE_READY, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+              if (it > 0 && !lap_wait(bar(LAP_O_FREE, pst), ppar, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+              tc_fence_after_sync();
+              for (int kq = 0; kq < nk16; ++kq) {  // X = A State
+                const uint32_t offA = (kq >> 2) * SLAB + (kq & 3) * 32;
+                if constexpr (WIDE) {
+                  umma_f16(tmem + T_OX, smem_desc_sw128(sAs + offA, 16), smem_desc_sw128(sS + kq * 2048, SLAB), IDESC_PC, kq > 0);
+                } else {
+                  const uint32_t offS = (kq >> 2) * (DV * 128) + (kq & 3) * 32;
+                  umma_f16(tmem + T_OX, smem_desc_sw128(sAs + offA, 16), smem_desc_sw128(sS + offS, 16), IDESC_X, kq > 0);
+                }
               }
             }
+            if (WIDE) umma_commit(bar(LAP_A_FREE, st));  // S and X of this block are done with A
+            LAP_TRACE(1, it)
           }
-          if (WIDE) umma_commit(bar(LAP_A_FREE, st));  // S and X of this block are done with A
-          LAP_TRACE(1, it)
-        }
-        if (MODE != 0 && !lap_wait(bar(LAP_FULL_AB, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_INPUT) break; }
-        if (!lap_wait(bar(LAP_FULL_C, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_INPUT) break; }
-        if (!lap_wait(bar(LAP_BM_SCALED, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
-        if (it > 0 && !lap_wait(bar(LAP_D_FREE, pst), ppar, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
-        tc_fence_after_sync();
-        if constexpr (WIDE) {
-#pragma unroll
-          for (int kk = 0; kk < 16; ++kk)  // local State = (w_state Bm)^T C, dk rows 0-127 and 128-255
-            umma_f16(tmem + T_D + (kk >> 3) * DV, smem_desc_sw128(sBs + (kk >> 3) * 2 * SLAB + (kk & 7) * 2048, SLAB),
-                     smem_desc_sw128(sCs + (kk & 7) * 2048, SLAB), IDESC_ST, (kk & 7) > 0);
-        } else {
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk)  // local StateT = C^T (w_state Bm)
-            umma_f16(tmem + T_D, smem_desc_sw128(sCs + kk * 2048, SLAB), smem_desc_sw128(sBs + kk * 2048, SLAB), IDESC_ST, kk > 0);
-        }
-        umma_commit(bar(LAP_D_DONE, st));  // also: X_it is done with the bf16 state copy
-        LAP_TRACE(3, it)
-        if (MODE == 0) {
-          if (!lap_wait(bar(LAP_P_READY, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
-          LAP_TRACE(2, it)
+          if (MODE != 0 && !lap_wait(bar(LAP_FULL_AB, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_INPUT) break; }
+          if (!lap_wait(bar(LAP_FULL_C, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_INPUT) break; }
+          if (!lap_wait(bar(LAP_BM_SCALED, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+          if (it > 0 && !lap_wait(bar(LAP_D_FREE, pst), ppar, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
           tc_fence_after_sync();
+          if constexpr (WIDE) {
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)  // O_intra = P C, P read from TMEM
-            umma_f16_ts(tmem + T_OI, tmem + T_S + kk * 8, smem_desc_sw128(sCs + kk * 2048, SLAB), IDESC_PC, kk > 0);
-          umma_commit(bar(LAP_PC_DONE, st));  // O_intra and O_inter are complete; nothing reads A, Bm, C of this block any more
-          if (it + 1 < nb) {
-            if (!issue_S(it + 1)) { LAP_FAIL(LA_ERR_WAIT_INPUT) break; }
+            for (int kk = 0; kk < 16; ++kk)  // local State = (w_state Bm)^T C, dk rows 0-127 and 128-255
+              umma_f16(tmem + T_D + (kk >> 3) * DV, smem_desc_sw128(sBs + (kk >> 3) * 2 * SLAB + (kk & 7) * 2048, SLAB),
+                       smem_desc_sw128(sCs + (kk & 7) * 2048, SLAB), IDESC_ST, (kk & 7) > 0);
+          } else {
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)  // local StateT = C^T (w_state Bm)
+              umma_f16(tmem + T_D, smem_desc_sw128(sCs + kk * 2048, SLAB), smem_desc_sw128(sBs + kk * 2048, SLAB), IDESC_ST, kk > 0);
+          }
+          umma_commit(bar(LAP_D_DONE, st));  // also: X_it is done with the bf16 state copy
+          LAP_TRACE(3, it)
+          if (MODE == 0) {
+            if (!lap_wait(bar(LAP_P_READY, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+            LAP_TRACE(2, it)
+            tc_fence_after_sync();
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)  // O_intra = P C, P read from TMEM
+              umma_f16_ts(tmem + T_OI, tmem + T_S + kk * 8, smem_desc_sw128(sCs + kk * 2048, SLAB), IDESC_PC, kk > 0);
+            umma_commit(bar(LAP_PC_DONE, st));  // O_intra and O_inter are complete; nothing reads A, Bm, C of this block any more
+            if (it + 1 < nb) {
+              if (!issue_S(it + 1)) { LAP_FAIL(LA_ERR_WAIT_INPUT) break; }
+            }
           }
         }
       }
     }
-  } else if (warp < 6) {
+  } else if (warp < 8) {
+    regs_set<128, LAP_REGS[1]>();
     // ============================================ mask group ============================================
     // One warp per TMEM lane quadrant, four 32-column tiles each, in column order. P tile t goes back into TMEM at
     // columns [16 t, 16 t + 16), i.e. over S columns of S tile t/2 <= t, which the warp has already pulled into
@@ -391,7 +401,8 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else {
     // ========================================= state / output group =====================================
-    const int w8 = warp - 6;
+    regs_set<128, LAP_REGS[2]>();
+    const int w8 = warp - 8;
     const int q = warp & 3, hf = w8 >> 2;
     const int r = q * 32 + lane;
     const uint32_t lanebase = static_cast<uint32_t>(q * 32) << 16;

@@ -139,6 +139,16 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// Register split between warpgroups: every warp of the warpgroup executes it, N the registers per thread it goes on with. The block
+// is launched with LAUNCHED per thread; setmaxnreg.inc takes only counts above the current one and .dec only counts below it
+// (the other way round is an illegal instruction), so the form is chosen here and an equal count issues neither.
+template <int LAUNCHED, int N>
+__device__ __forceinline__ void regs_set() {
+  static_assert(N % 8 == 0 && N >= 24 && N <= 255, "setmaxnreg range");
+  if constexpr (N > LAUNCHED) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+  if constexpr (N < LAUNCHED) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 // Shared-memory matrix descriptor, 128-byte swizzle, tile rows of 128 bytes (64 16-bit elements),
 // 8-row groups 1024 bytes apart.
 //   K-major operand  (contraction runs along the 128-byte rows): LBO unused.
