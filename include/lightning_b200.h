@@ -182,6 +182,16 @@ int lab200_la2_bwd(const void* q, const void* k, const void* v, const float* slo
                    void* dq, void* dk, void* dv, void* workspace, size_t workspace_bytes, int b, int h,
                    int n, int d, int e, int chunks, int dtype, void* stream);
 
+/*
+ * lab200_la2_bwd for d == e after a lab200_la2_fwd (or lab200_la_generic on (q, k, v) without state_in) of the same problem whose
+ * workspace, `kept`, has been left alone since: dq takes its chunk states over instead of computing them again. The states are read, not changed.
+ * Only where the library cuts the sequence into chunks (lab200_la_plan_chunks > 1), else LAB200_ERR_SHAPE. `workspace` is the
+ * call's own, lab200_la2_bwd_workspace_bytes. No counterpart in the reference.
+ */
+int lab200_la2_bwd_kept(const void* q, const void* k, const void* v, const float* slopes, const void* dout, void* dq, void* dk,
+                        void* dv, void* kept, size_t kept_bytes, void* workspace, size_t workspace_bytes, int b, int h, int n,
+                        int d, int chunks, int dtype, void* stream);
+
 /* Bytes of workspace lab200_la2_bwd needs: the largest need of the three products it runs ((dk, dv) = (e, d) for dq
  * and for dk/dv, (d, e) for dv on the unfused path), each with its own chunk plan when `chunks` = 0. */
 size_t lab200_la2_bwd_workspace_bytes(int b, int h, int n, int d, int e, int chunks);

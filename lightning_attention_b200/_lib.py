@@ -61,6 +61,8 @@ def lib():
         L.lab200_la2_bwd_workspace_bytes.argtypes = [i, i, i, i, i, i]
         L.lab200_la2_bwd.restype = i
         L.lab200_la2_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, sz, i, i, i, i, i, i, i, vp]
+        L.lab200_la2_bwd_kept.restype = i
+        L.lab200_la2_bwd_kept.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp, sz, i, i, i, i, i, i, vp]
         L.lab200_last_status.restype = i
         L.lab200_last_status.argtypes = []
         L.lab200_static_status.restype = i
@@ -79,8 +81,7 @@ def lib():
 
 _host = None
 _HOST_ENTRIES = ("lab200_error_string", "lab200_last_status", "lab200_la_plan_chunks", "lab200_la_workspace_bytes", "lab200_la_generic",
-                 "lab200_la_generic_resume_swapped", "lab200_la_decode_step", "lab200_la2_fwd", "lab200_la2_bwd",
-                 "lab200_la2_bwd_workspace_bytes", "lab200_la2_dkdv", "lab200_srmsnorm_fwd", "lab200_srmsnorm_bwd",
+                 "lab200_la_decode_step", "lab200_la2_fwd", "lab200_la2_bwd", "lab200_la2_bwd_workspace_bytes", "lab200_la2_bwd_kept", "lab200_srmsnorm_fwd", "lab200_srmsnorm_bwd",
                  "lab200_srmsnorm_gate_fwd", "lab200_srmsnorm_gate_bwd")
 
 
@@ -101,7 +102,7 @@ def host():
 
 EXPORTS = [
     "lab200_version", "lab200_launch_count", "lab200_la_debug_trace", "lab200_error_string", "lab200_la_plan_chunks", "lab200_la_workspace_bytes",
-    "lab200_la_generic", "lab200_la_generic_resume", "lab200_la_generic_resume_swapped", "lab200_la_combine_states", "lab200_la_decode_step", "lab200_la2_fwd", "lab200_la2_fwd_static", "lab200_la2_bwd", "lab200_la2_bwd_workspace_bytes", "lab200_la2_dkdv", "lab200_read_status", "lab200_last_status", "lab200_static_status", "lab200_debug_wait_expiry",
+    "lab200_la_generic", "lab200_la_generic_resume", "lab200_la_generic_resume_swapped", "lab200_la_combine_states", "lab200_la_decode_step", "lab200_la2_fwd", "lab200_la2_fwd_static", "lab200_la2_bwd", "lab200_la2_bwd_workspace_bytes", "lab200_la2_bwd_kept", "lab200_la2_dkdv", "lab200_read_status", "lab200_last_status", "lab200_static_status", "lab200_debug_wait_expiry",
     "lab200_srmsnorm_fwd", "lab200_srmsnorm_bwd", "lab200_srmsnorm_gate_fwd", "lab200_srmsnorm_gate_bwd",
 ]
 

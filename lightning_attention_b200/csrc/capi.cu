@@ -201,7 +201,9 @@ int la_validate(const void* a, const void* bm, const void* c, const void* out, c
 // The generic product without the status reset (so that composite calls share one status word).
 // PREFIX_ONLY: stop once the state entering every chunk is in the workspace (computed, or with RESUME taken over from
 // an earlier call and rebased); the block loop is the caller's business (the fused dk+dv sweep). a and out may be null.
-enum : int { RESUME = 1, RESUME_SWAPPED = 2, RESUME_NO_REBASE = 4, PREFIX_ONLY = 8 };
+// RESUME_SWAPPED transposes the kept states in place, as callers that go on with them expect; RESUME_READ_SWAPPED has the block loop
+// read them transposed and leaves them as they are (without the transposing launch: 4.6-6.8 us and the gap).
+enum : int { RESUME = 1, RESUME_SWAPPED = 2, RESUME_NO_REBASE = 4, PREFIX_ONLY = 8, RESUME_READ_SWAPPED = 16 };
 
 // Number of chunks la_generic_impl cuts the sequence into.
 int chunk_count(int bh, int n, int dk, int dv, int chunks) {
@@ -247,6 +249,7 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
   p.nblocks = nblocks;
   p.blocks_per_chunk = bpc;
   p.reverse = reverse ? 1 : 0;
+  p.in_swapped = 0;
   p.layout = layout;
   p.wait_budget = WAIT_BUDGET;
   p.trace = g_trace.load(std::memory_order_relaxed);
@@ -268,8 +271,8 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
     // the workspace already holds the per-chunk prefix states of a preceding call: go straight to the block loop.
     // RESUME_SWAPPED: they belong to the product with Bm and C exchanged, i.e. they are the transposes (dk == dv).
     // Unless RESUME_NO_REBASE is set they were computed from a zero initial state and the decayed incoming state is added.
+    if ((resume & (RESUME_SWAPPED | RESUME_READ_SWAPPED)) && dk != dv) return LAB200_ERR_SHAPE;
     if (resume & RESUME_SWAPPED) {
-      if (dk != dv) return LAB200_ERR_SHAPE;
       const int nt = (dk + 31) / 32;
       la_transpose_square_kernel<<<dim3(static_cast<unsigned>(bh) * nchunks, nt * (nt + 1) / 2), dim3(32, 8), 0, st>>>(states, dk);
       g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -284,6 +287,7 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
       if (cudaGetLastError() != cudaSuccess) return LAB200_ERR_CUDA;
     }
     if (prefix_only) return LAB200_OK;
+    p.in_swapped = (resume & RESUME_READ_SWAPPED) ? 1 : 0;
     p.state_slots = nchunks;
     p.chunk0 = 0;
     p.state_in = states;
@@ -832,10 +836,35 @@ int lab200_la2_bwd(const void* q, const void* k, const void* v, const float* slo
                        chunks, dtype, st, status);
   if (rc != LAB200_OK) return rc;
   // In chunk mode the dk launch leaves the reverse-time state entering every chunk, sum lambda^t q_t^T do_t as (d, e), in
-  // the workspace; dv needs the same states as (e, d). With d == e they are transposed in place instead of recomputed.
-  const int resume = (d == e && chunk_count(bh, n, e, d, chunks) > 1) ? (RESUME | RESUME_SWAPPED | RESUME_NO_REBASE) : 0;
+  // the workspace; dv needs the same states as (e, d). With d == e they are read transposed instead of being recomputed.
+  const int resume = (d == e && chunk_count(bh, n, e, d, chunks) > 1) ? (RESUME | RESUME_READ_SWAPPED | RESUME_NO_REBASE) : 0;
   return la_generic_impl(k, q, dout, slopes, dv, nullptr, nullptr, workspace, workspace_bytes, bh, h, n, d, e, 1, 0,
                          chunks, dtype, st, status, resume);
+}
+
+int lab200_la2_bwd_kept(const void* q, const void* k, const void* v, const float* slopes, const void* dout, void* dq, void* dk,
+                        void* dv, void* kept, size_t kept_bytes, void* workspace, size_t workspace_bytes, int b, int h, int n,
+                        int d, int chunks, int dtype, void* stream) {
+  if (b < 1 || h < 1 || b > 65535 / h) return LAB200_ERR_SHAPE;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int bh = b * h;
+  int rc = la_validate(dout, v, k, dq, nullptr, nullptr, kept, bh, h, n, d, d, 0, dtype);
+  if (rc == LAB200_OK) rc = la_validate(k, q, dout, dv, nullptr, nullptr, workspace, bh, h, n, d, d, 0, dtype);
+  if (rc == LAB200_OK && (!q || !dk || !aligned16(q) || !aligned16(dk))) rc = q && dk ? LAB200_ERR_ALIGN : LAB200_ERR_SHAPE;
+  if (rc != LAB200_OK) return rc;
+  if (chunk_count(bh, n, d, d, chunks) < 2) return LAB200_ERR_SHAPE;  // nothing was kept
+  if (!workspace_ok(workspace, workspace_bytes) || !workspace_ok(kept, kept_bytes)) return LAB200_ERR_WORKSPACE;
+  CallStatus status(workspace, host_status_word(true));
+  if ((rc = la_generic_impl(dout, v, k, slopes, dq, nullptr, nullptr, kept, kept_bytes, bh, h, n, d, d, 0, 0, chunks, dtype, st, status,
+                            RESUME | RESUME_READ_SWAPPED | RESUME_NO_REBASE)) != LAB200_OK)
+    return rc;
+  if (dkdv_shape_ok(d, d))
+    return la_dkdv_full(q, k, v, dout, slopes, dk, dv, nullptr, workspace, workspace_bytes, bh, h, n, d, d, chunks, 0, dtype, st, status);
+  if ((rc = la_generic_impl(v, dout, q, slopes, dk, nullptr, nullptr, workspace, workspace_bytes, bh, h, n, d, d, 1, 0, chunks, dtype, st,
+                            status)) != LAB200_OK)
+    return rc;
+  return la_generic_impl(k, q, dout, slopes, dv, nullptr, nullptr, workspace, workspace_bytes, bh, h, n, d, d, 1, 0, chunks, dtype, st, status,
+                         RESUME | RESUME_READ_SWAPPED | RESUME_NO_REBASE);
 }
 
 size_t lab200_la2_bwd_workspace_bytes(int b, int h, int n, int d, int e, int chunks) {

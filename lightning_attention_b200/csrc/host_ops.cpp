@@ -26,12 +26,11 @@ struct Api {
   decltype(&lab200_la_plan_chunks) plan_chunks;
   decltype(&lab200_la_workspace_bytes) workspace_bytes;
   decltype(&lab200_la_generic) generic;
-  decltype(&lab200_la_generic_resume_swapped) resume_swapped;
   decltype(&lab200_la_decode_step) decode_step;
   decltype(&lab200_la2_fwd) la2_fwd;
   decltype(&lab200_la2_bwd) la2_bwd;
   decltype(&lab200_la2_bwd_workspace_bytes) la2_bwd_workspace_bytes;
-  decltype(&lab200_la2_dkdv) la2_dkdv;
+  decltype(&lab200_la2_bwd_kept) la2_bwd_kept;
   decltype(&lab200_srmsnorm_fwd) srms_fwd;
   decltype(&lab200_srmsnorm_bwd) srms_bwd;
   decltype(&lab200_srmsnorm_gate_fwd) gate_fwd;
@@ -53,12 +52,11 @@ void bind(const std::unordered_map<std::string, uintptr_t>& t) {
   set_entry(t, "lab200_la_plan_chunks", a.plan_chunks);
   set_entry(t, "lab200_la_workspace_bytes", a.workspace_bytes);
   set_entry(t, "lab200_la_generic", a.generic);
-  set_entry(t, "lab200_la_generic_resume_swapped", a.resume_swapped);
   set_entry(t, "lab200_la_decode_step", a.decode_step);
   set_entry(t, "lab200_la2_fwd", a.la2_fwd);
   set_entry(t, "lab200_la2_bwd", a.la2_bwd);
   set_entry(t, "lab200_la2_bwd_workspace_bytes", a.la2_bwd_workspace_bytes);
-  set_entry(t, "lab200_la2_dkdv", a.la2_dkdv);
+  set_entry(t, "lab200_la2_bwd_kept", a.la2_bwd_kept);
   set_entry(t, "lab200_srmsnorm_fwd", a.srms_fwd);
   set_entry(t, "lab200_srmsnorm_bwd", a.srms_bwd);
   set_entry(t, "lab200_srmsnorm_gate_fwd", a.gate_fwd);
@@ -139,7 +137,7 @@ const float* float_ptr(const Tensor& s) { return s.defined() ? static_cast<const
 
 // ---- attention -------------------------------------------------------------------------------------------------------------
 // Same protocol as LightningAttention2 / LightningAttention2NoDecay in lightning_attn2.py: where the library cuts the sequence into
-// chunks and d == e, the forward pass keeps its workspace, whose chunk states the first backward pass takes over transposed.
+// chunks and d == e, the forward pass keeps its workspace, and the first backward pass reads its chunk states transposed.
 struct Attention : torch::autograd::Function<Attention> {
   static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<Tensor>& s_opt, bool bnhd) {
     const Tensor s = s_opt.has_value() ? *s_opt : Tensor();
@@ -161,7 +159,7 @@ struct Attention : torch::autograd::Function<Attention> {
     const variable_list saved = ctx->get_saved_variables();
     const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &s = saved[3];
     const bool bnhd = ctx->saved_data["bnhd"].toBool();
-    Tensor kept;  // usable once: the transposed hand-over changes whose states they are
+    Tensor kept;  // given back with the first backward pass; a second one computes its states again
     const auto it = ctx->saved_data.find("kept");
     if (it != ctx->saved_data.end()) {
       kept = it->second.toTensor();
@@ -178,26 +176,13 @@ struct Attention : torch::autograd::Function<Attention> {
     const float* sl = float_ptr(s);
     const void *qp = q.const_data_ptr(), *kp = k.const_data_ptr(), *vp = v.const_data_ptr(), *gp = go.const_data_ptr();
     void *dqp = dq.mutable_data_ptr(), *dkp = dk.mutable_data_ptr(), *dvp = dv.mutable_data_ptr(), *st = stream_of(q);
-    const int bh = z.b * z.h;
-    if (!kept.defined()) {
-      const size_t bytes = g_api.la2_bwd_workspace_bytes(z.b, z.h, z.n, z.d, z.e, 0);
-      Tensor ws = workspace(bytes, q);
-      check(g_api.la2_bwd(qp, kp, vp, sl, gp, dqp, dkp, dvp, ws.mutable_data_ptr(), bytes, z.b, z.h, z.n, z.d, z.e, 0, z.dt, st), "lab200_la2_bwd");
+    const size_t bytes = g_api.la2_bwd_workspace_bytes(z.b, z.h, z.n, z.d, z.e, 0);
+    Tensor ws = workspace(bytes, q);
+    if (kept.defined()) {
+      check(g_api.la2_bwd_kept(qp, kp, vp, sl, gp, dqp, dkp, dvp, kept.mutable_data_ptr(), kept.numel(), ws.mutable_data_ptr(), bytes, z.b, z.h,
+                               z.n, z.d, 0, z.dt, st), "lab200_la2_bwd_kept");
     } else {
-      const size_t bytes = kept.numel();
-      // d == e, so every product of this problem has the same workspace size and chunk plan
-      check(g_api.resume_swapped(gp, vp, kp, sl, dqp, nullptr, kept.mutable_data_ptr(), bytes, bh, z.h, z.n, z.d, z.d, 0, 0, 0, z.dt, st),
-            "lab200_la_generic_resume");
-      Tensor ws = workspace(bytes, q);
-      if (z.d <= 128) {
-        check(g_api.la2_dkdv(qp, kp, vp, sl, gp, dkp, dvp, nullptr, ws.mutable_data_ptr(), bytes, z.b, z.h, z.n, z.d, z.e, 0, 0, z.dt, st),
-              "lab200_la2_dkdv");
-      } else {
-        check(g_api.generic(vp, gp, qp, sl, dkp, nullptr, nullptr, ws.mutable_data_ptr(), bytes, bh, z.h, z.n, z.d, z.d, 1, 0, 0, z.dt, st),
-              "lab200_la_generic");
-        check(g_api.resume_swapped(kp, qp, gp, sl, dvp, nullptr, ws.mutable_data_ptr(), bytes, bh, z.h, z.n, z.d, z.d, 1, 0, 0, z.dt, st),
-              "lab200_la_generic_resume");
-      }
+      check(g_api.la2_bwd(qp, kp, vp, sl, gp, dqp, dkp, dvp, ws.mutable_data_ptr(), bytes, z.b, z.h, z.n, z.d, z.e, 0, z.dt, st), "lab200_la2_bwd");
     }
     return {dq, dk, dv, Tensor(), Tensor()};
   }

@@ -73,6 +73,7 @@ struct LaParams {
   const float* slopes;     // [h] decay rates, or nullptr for no decay
   const float* state_in;   // [bh][state_slots][dv][dk] fp32, or nullptr for a zero initial state
   float* state_out;        // same indexing, or nullptr
+  int in_swapped;          // the matrices of state_in are stored [dk][dv]: they come from the product with Bm and C exchanged (block loop)
   LaStatus status;         // where a failure is reported
   int n, h, dk, dv;
   int nblocks;             // ceil(n / 128)

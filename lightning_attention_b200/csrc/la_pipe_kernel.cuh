@@ -35,19 +35,23 @@ static_assert(LAP_REGS[0] + LAP_REGS[1] + 2 * LAP_REGS[2] <= 512, "the split mus
 constexpr int LAP_MASK_THREADS = 128, LAP_STATE_THREADS = 256;
 
 
-// barrier slots (each has two instances, indexed by block parity)
+// barrier slots (each has one instance per stage, indexed by block modulo the stage count)
 enum : int { LAP_FULL_AB = 0, LAP_FULL_C, LAP_S_READY, LAP_P_READY, LAP_PC_DONE, LAP_D_DONE, LAP_O_FREE, LAP_D_FREE,
              LAP_STATE_READY, LAP_O_STAGED, LAP_BM_SCALED, LAP_A_FREE, LAP_NUM_BARS };
 
 // Shared-memory stages, in 16 KB slabs (host and device agree through these).
 __host__ __device__ constexpr bool lap_wide(int nks) { return nks > 2; }
 __host__ __device__ constexpr int lap_a_slabs(int nks, int nvs) { return lap_wide(nks) ? nks : 2 * (nks > nvs ? nks : nvs); }  // all stages of A, full block loop
-__host__ __device__ constexpr int lap_b_stages(int nks, int mode) { return (nks == 4 && mode == 0) ? 1 : 2; }
+// Two stages in the full block loop. The state-only pass has nothing else in shared memory and takes three of (Bm, C), as far as they
+// fit: a stage goes through load, scaling and D before its reload, and two of them left HBM idle between (b1 h32 n131072
+// d=e=128: 339 -> 311 us per pass, 6.9 TB/s; b2 h16 n4096: 22.6 -> 20.6).
+__host__ __device__ constexpr int lap_stages(int mode, int nks) { return (mode == 0 || nks == 4) ? 2 : 3; }
+__host__ __device__ constexpr int lap_b_stages(int nks, int mode) { return (nks == 4 && mode == 0) ? 1 : lap_stages(mode, nks); }
 __host__ __device__ constexpr int lap_c_slabs(int nks) { return lap_wide(nks) ? 1 : 2; }  // per stage: the M = 128 side of D for dk <= 128 reads two
 __host__ __device__ constexpr int lap_smem_bytes(int nks, int nvs, int mode) {
-  int b = (lap_b_stages(nks, mode) * nks + 2 * lap_c_slabs(nks)) * LA_SLAB_BYTES;
+  int b = (lap_b_stages(nks, mode) * nks + lap_stages(mode, nks) * lap_c_slabs(nks)) * LA_SLAB_BYTES;
   if (mode == 0) b += lap_a_slabs(nks, nvs) * LA_SLAB_BYTES + nks * nvs * 64 * 128;
-  return b + 2 * LAP_NUM_BARS * 8 + 16 + 512 + 1024;  // barriers, flags, decay table, alignment slack
+  return b + lap_stages(mode, nks) * LAP_NUM_BARS * 8 + 16 + 512 + 1024;  // barriers, flags, decay table, alignment slack
 }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -95,7 +99,8 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   constexpr int SC = WIDE ? DV : DKP / 2;  // state columns per thread
   constexpr int OC = DV / 2;
   constexpr int NAS = WIDE ? 0 : (NKS > NVS ? NKS : NVS);  // slabs from one A stage to the next (0: there is one)
-  constexpr int NBS = lap_b_stages(NKS, MODE) == 2 ? NKS : 0;
+  constexpr int NBS = lap_b_stages(NKS, MODE) > 1 ? NKS : 0;
+  constexpr int NST = lap_stages(MODE, NKS);
   constexpr int NCS = lap_c_slabs(NKS);
   constexpr uint32_t T_S = 0, T_OI = 128, T_OX = 128 + DV, T_D = 128 + 2 * DV;
   static_assert(T_D + (WIDE ? 2 * DV : DKP) <= 512, "TMEM budget");
@@ -113,15 +118,19 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // 16-bit state: NKS x [DV rows][128 B] (rows dv, columns dk); wide: [DKP rows][128 B] (rows dk, columns dv) (MODE 0). The second
   // M = 128 tile of D at NKS = 3 reads one slab behind its Bm stage: that is the other stage or C, and only reaches accumulator
   // rows that nobody reads.
-  const uint32_t sS = sC + 2 * NCS * SLAB;
+  const uint32_t sS = sC + NST * NCS * SLAB;
   // Output tiles are staged in the C stage of their own block (free once P C is done) and leave by TMA store.
   const uint32_t sBar = sS + (MODE == 0 ? NKS * DV * 128 : 0);      // 2 x LAP_NUM_BARS mbarriers
-  const uint32_t sMisc = sBar + 2 * LAP_NUM_BARS * 8;
+  const uint32_t sMisc = sBar + NST * LAP_NUM_BARS * 8;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_raw + (sMisc - raw));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_raw + (sMisc + 4 - raw));
   volatile int* fail_code = reinterpret_cast<volatile int*>(smem_raw + (sMisc + 8 - raw));
   volatile float* decay_tab = reinterpret_cast<volatile float*>(smem_raw + (sMisc + 16 - raw));
-  auto bar = [&](int which, int inst) -> uint32_t { return sBar + (which * 2 + inst) * 8; };
+  auto bar = [&](int which, int inst) -> uint32_t { return sBar + (which * NST + inst) * 8; };
+  auto stage_of = [](int i) { return NST == 2 ? (i & 1) : i % NST; };                       // stage and barrier instance of block i
+  auto parity_of = [](int i) -> uint32_t { return (NST == 2 ? (i >> 1) : i / NST) & 1; };  // and the barriers' phase
+  // accumulator of D: the state-only pass alternates between two, so that D of a block does not wait for the readers of the last
+  auto t_d = [](int i) -> uint32_t { return MODE == 0 ? T_D : T_D - ((i & 1) ? 256u : 0u); };
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
@@ -147,8 +156,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     for (int i = 0; i < LAP_NUM_BARS; ++i) {
       const uint32_t count = (i == LAP_P_READY) ? LAP_MASK_THREADS
                            : (i == LAP_O_FREE || i == LAP_D_FREE || i == LAP_STATE_READY || i == LAP_O_STAGED || i == LAP_BM_SCALED) ? LAP_STATE_THREADS : 1u;
-      mbar_init(bar(i, 0), count);
-      mbar_init(bar(i, 1), count);
+      for (int j = 0; j < NST; ++j) mbar_init(bar(i, j), count);
     }
     *abort_flag = 0;
     *fail_code = 0;
@@ -192,18 +200,18 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         bool alive = true;
         for (int it = 0; it < nb && alive; ++it) {
           const int blk = blk_of(it);
-          const int st = it & 1;
-          const uint32_t prev_par = ((it >> 1) & 1) ^ 1;  // parity of the previous use of this stage (block it-2)
+          const int st = stage_of(it);
+          const uint32_t prev_par = parity_of(it) ^ 1;  // phase of the previous use of this stage (block it - NST)
           // A and Bm of block it: their stages are free once every MMA of block it-2 has run (P C is the last one issued; in
           // state-only mode D). They are what S of block it waits for, so they go first and wait for nothing else.
           // Where there is one stage, A is free after X of block it-1 and Bm after D of block it-1.
-          const uint32_t last_par = ((it - 1) >> 1) & 1;
+          const uint32_t last_par = parity_of(it - 1);
           auto load_b = [&]() {
 #pragma unroll
             for (int ks = 0; ks < NKS; ++ks)
               tma_load_3d(sB + (st * NBS + ks) * SLAB, &tmB, ks * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_AB, st));
           };
-          if (NBS != 0 && it >= 2) {
+          if (NBS != 0 && it >= NST) {
             if (!lap_wait(bar(MODE == 0 ? LAP_PC_DONE : LAP_D_DONE, st), prev_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
           }
           mbar_arrive_expect_tx(bar(LAP_FULL_AB, st), (MODE == 0 ? 2 * NKS : NKS) * SLAB);
@@ -264,10 +272,10 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if (!alive) LAP_FAIL(LA_ERR_WAIT_INPUT)
         }
         for (int it = 0; it < nb && alive; ++it) {
-          const int st = it & 1;
-          const uint32_t par = (it >> 1) & 1;
-          const int pst = st ^ 1;                         // instance used by block it-1
-          const uint32_t ppar = ((it - 1) >> 1) & 1;      // and its parity
+          const int st = stage_of(it);
+          const uint32_t par = parity_of(it);
+          const int pst = stage_of(it - 1);               // instance used by block it-1
+          const uint32_t ppar = parity_of(it - 1);        // and its phase
           const uint32_t sAs = sA + st * NAS * SLAB, sBs = sB + st * NBS * SLAB, sCs = sC + st * NCS * SLAB;
           const bool have_state = have_state_in || (it > 0);
           LAP_TRACE(0, it)
@@ -292,17 +300,21 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if (MODE != 0 && !lap_wait(bar(LAP_FULL_AB, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_INPUT) break; }
           if (!lap_wait(bar(LAP_FULL_C, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_INPUT) break; }
           if (!lap_wait(bar(LAP_BM_SCALED, st), par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
-          if (it > 0 && !lap_wait(bar(LAP_D_FREE, pst), ppar, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+          if (MODE == 0) {
+            if (it > 0 && !lap_wait(bar(LAP_D_FREE, pst), ppar, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
+          } else if (it > 1 && !lap_wait(bar(LAP_D_FREE, stage_of(it - 2)), parity_of(it - 2), abort_flag, budget)) {
+            LAP_FAIL(LA_ERR_WAIT_MMA2) break;
+          }
           tc_fence_after_sync();
           if constexpr (WIDE) {
 #pragma unroll
             for (int kk = 0; kk < 16; ++kk)  // local State = (w_state Bm)^T C, dk rows 0-127 and 128-255
-              umma_f16(tmem + T_D + (kk >> 3) * DV, smem_desc_sw128(sBs + (kk >> 3) * 2 * SLAB + (kk & 7) * 2048, SLAB),
+              umma_f16(tmem + t_d(it) + (kk >> 3) * DV, smem_desc_sw128(sBs + (kk >> 3) * 2 * SLAB + (kk & 7) * 2048, SLAB),
                        smem_desc_sw128(sCs + (kk & 7) * 2048, SLAB), IDESC_ST, (kk & 7) > 0);
           } else {
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)  // local StateT = C^T (w_state Bm)
-              umma_f16(tmem + T_D, smem_desc_sw128(sCs + kk * 2048, SLAB), smem_desc_sw128(sBs + kk * 2048, SLAB), IDESC_ST, kk > 0);
+              umma_f16(tmem + t_d(it), smem_desc_sw128(sCs + kk * 2048, SLAB), smem_desc_sw128(sBs + kk * 2048, SLAB), IDESC_ST, kk > 0);
           }
           umma_commit(bar(LAP_D_DONE, st));  // also: X_it is done with the bf16 state copy
           LAP_TRACE(3, it)
@@ -428,16 +440,18 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     for (int i = 0; i < SC; ++i) stt[i] = 0.f;
     if (have_state_in && st_row_valid) {
       const float* src = p.state_in + (static_cast<size_t>(bh) * p.state_slots + chunk) * p.dv * p.dk;
-      if constexpr (WIDE) {  // neighbouring lanes read neighbouring dk
-        src += static_cast<size_t>(dv_off) * p.dk + st_row;
+      const bool swapped = MODE == 0 && p.in_swapped;
+      const int ld = swapped ? p.dv : p.dk, cols = WIDE ? p.dv - dv_off : p.dk - hf * SC;
+      if (WIDE != swapped) {  // this thread's part is a column of the stored matrix: neighbouring lanes read neighbouring elements
+        src += WIDE ? static_cast<size_t>(dv_off) * ld + st_row : static_cast<size_t>(hf * SC) * ld + dv_off + r;
 #pragma unroll
         for (int i = 0; i < SC; ++i)
-          if (dv_off + i < p.dv) stt[i] = src[static_cast<size_t>(i) * p.dk];
+          if (i < cols) stt[i] = src[static_cast<size_t>(i) * ld];
       } else {
-        src += static_cast<size_t>(dv_off + r) * p.dk + hf * SC;
+        src += WIDE ? static_cast<size_t>(st_row) * ld + dv_off : static_cast<size_t>(dv_off + r) * ld + hf * SC;
 #pragma unroll
         for (int i = 0; i < SC; i += 4) {
-          if (hf * SC + i < p.dk) {
+          if (i < cols) {
             const float4 v4 = *reinterpret_cast<const float4*>(src + i);
             stt[i] = v4.x; stt[i + 1] = v4.y; stt[i + 2] = v4.z; stt[i + 3] = v4.w;
           }
@@ -465,9 +479,9 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     // Bm rows of block j *= w_state(r), in place, for D_j: this thread's half of the row's 16-byte chunks.
     auto scale_bm = [&](int j) -> bool {
-      const int st = j & 1;
+      const int st = stage_of(j);
       // S_j must be done with the unscaled tile (state-only mode: the tile must have landed)
-      bool ok = lap_wait(bar(MODE == 0 ? LAP_S_READY : LAP_FULL_AB, st), (j >> 1) & 1, abort_flag, budget);
+      bool ok = lap_wait(bar(MODE == 0 ? LAP_S_READY : LAP_FULL_AB, st), parity_of(j), abort_flag, budget);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) return false;
       if (WIDE && s != 0.f) {
@@ -525,8 +539,8 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (!live) LAP_FAIL(LA_ERR_WAIT_MMA1)
     }
     for (int it = 0; it < nb && live; ++it) {
-      const int st = it & 1;
-      const uint32_t par = (it >> 1) & 1;
+      const int st = stage_of(it);
+      const uint32_t par = parity_of(it);
       const bool has_next = (it + 1 < nb);
       const bool have_state = have_state_in || (it > 0);
       // state-only mode: the next block's Bm tile is scaled while D of this block runs
@@ -543,7 +557,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
         for (int cc = 0; cc < SC; cc += 32) {
           uint32_t dl[32];
-          tmem_ld32(tmem + lanebase + T_D + hf * SC + cc, dl);
+          tmem_ld32(tmem + lanebase + t_d(it) + hf * SC + cc, dl);
           tmem_wait_ld();
 #pragma unroll
           for (int i = 0; i < 32; ++i)

@@ -547,6 +547,51 @@ def test_wide_keys_against_the_oracle(cuda_lib, n, dk, dv, chunks, reverse, dtyp
             assert O.rel_l2_err(f(only), want) <= tol
 
 
+@pytest.mark.parametrize("dk,dv", [(64, 64), (128, 128), (128, 64), (192, 64), (256, 128)])
+@pytest.mark.parametrize("n", [1, 128, 130, 384, 512, 900])
+def test_state_only_pass_over_few_blocks(cuda_lib, n, dk, dv):
+    """Fewer blocks than the pass has stages, as many, and more; both directions. Scaled rows are rounded once to bf16 (narrow
+    widths: with a bf16 factor, two more roundings), each at most 2^-9 relative."""
+    torch.manual_seed(42)
+    b, h = 1, 3
+    bm = torch.randn((b, h, n, dk), device=DEV).bfloat16()
+    c = torch.randn((b, h, n, dv), device=DEV).bfloat16()
+    s = (la._build_slope_tensor(h).reshape(-1) * 0.1).to(DEV)
+    f = lambda t: t.float().cpu().numpy()
+    for chunks in (1, 2):
+        st = c_generic(cuda_lib, None, bm, c, s, False, None, True, chunks, state_only=True)[1]
+        assert O.rel_l2_err(f(st), O.state_entering(f(bm), f(c), f(s))) <= 3 * 2.0 ** -9
+        if n % 128 == 0:
+            st = c_generic(cuda_lib, None, bm, c, s, True, None, True, chunks, state_only=True)[1]
+            assert O.rel_l2_err(f(st), O.la_generic(np.zeros((b, h, n, dk)), f(bm), f(c), f(s), reverse=True)[1]) <= 3 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("d", [64, 128, 192])
+@pytest.mark.parametrize("n,chunks", [(256, 2), (700, 3), (1300, 5)])
+def test_backward_from_kept_chunk_states(cuda_lib, d, n, chunks):
+    """lab200_la2_bwd_kept reads the forward's chunk states transposed and leaves them as they are; against lab200_la2_bwd, whose
+    chunk states are sums of the same bf16 products in another order (rounded copies may then differ by one bf16 step, 2^-8)."""
+    b, h = 1, 3
+    q, k, v, do = (t.detach() for t in make_inputs(b, h, n, d, d, torch.bfloat16, 1.0))
+    s = (la._build_slope_tensor(h).reshape(-1) * 0.1).to(DEV)
+    stream = torch.cuda.current_stream().cuda_stream
+    nbytes = cuda_lib.lab200_la2_bwd_workspace_bytes(b, h, n, d, d, chunks)
+    kept, ws = (torch.empty(nbytes, dtype=torch.uint8, device=DEV) for _ in range(2))
+    o, got, ref = torch.empty_like(v), [torch.empty_like(q) for _ in range(3)], [torch.empty_like(q) for _ in range(3)]
+    tail = (b, h, n, d, d, chunks, _lib.BF16, stream)
+    assert cuda_lib.lab200_la2_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), s.data_ptr(), o.data_ptr(), kept.data_ptr(), nbytes, *tail) == 0
+    before = kept.clone()
+    args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), s.data_ptr(), do.data_ptr())
+    outs = tuple(t.data_ptr() for t in got)
+    assert cuda_lib.lab200_la2_bwd_kept(*args, *outs, kept.data_ptr(), nbytes, ws.data_ptr(), nbytes, b, h, n, d, chunks, _lib.BF16, stream) == 0
+    assert cuda_lib.lab200_read_status(ws.data_ptr(), stream) == 0 and torch.equal(kept, before)
+    assert cuda_lib.lab200_la2_bwd(*args, *(t.data_ptr() for t in ref), ws.data_ptr(), nbytes, *tail) == 0
+    for x, y in zip(got, ref):
+        assert torch.linalg.vector_norm((x - y).float()) <= 2.0 ** -8 * torch.linalg.vector_norm(y.float())
+    one = (b, h, n, d, 1, _lib.BF16, stream)
+    assert cuda_lib.lab200_la2_bwd_kept(*args, *outs, kept.data_ptr(), nbytes, ws.data_ptr(), nbytes, *one) != 0
+
+
 def test_decode_step_against_numpy_oracle(cuda_lib):
     torch.manual_seed(23)
     b, h, d, e = 3, 5, 48, 80
