@@ -75,6 +75,25 @@ int make_tmap(CUtensorMap* tm, const void* ptr, int bh, int n, int dim, int dtyp
   return r == CUDA_SUCCESS ? LAB200_OK : LAB200_ERR_DRIVER;
 }
 
+// Launches a kernel of an attention call. `follows`: it comes behind another kernel of the same call and may start while that one
+// ends (see pdl_wait_for_previous). The first kernel of a call is an ordinary launch: what precedes the call need not know.
+template <class K, class... A>
+int launch_kernel(K kern, dim3 grid, unsigned threads, size_t smem, cudaStream_t st, bool follows, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = follows ? 1 : 0;
+  const cudaError_t rc = cudaLaunchKernelEx(&cfg, kern, args...);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return (rc == cudaSuccess && cudaGetLastError() == cudaSuccess) ? LAB200_OK : LAB200_ERR_CUDA;
+}
+
 struct Tiling {
   int nks, nvs, nslices;
 };
@@ -112,9 +131,7 @@ int launch_pipe_one(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensor
     cudaGetLastError();
     return LAB200_ERR_CUDA;
   }
-  kern<<<grid, LAP_THREADS, smem, st>>>(tA, tB, tC, tO, p);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? LAB200_OK : LAB200_ERR_CUDA;
+  return launch_kernel(kern, grid, LAP_THREADS, smem, st, !p.status.reset, tA, tB, tC, tO, p);
 }
 
 template <int MODE, int FMT>
@@ -314,11 +331,10 @@ int la_generic_impl(const void* a, const void* bm, const void* c, const float* s
 
   const int elems4 = dv * dk / 4;
   const long long total = static_cast<long long>(bh) * elems4;
-  la_scan_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, st>>>(
-      reinterpret_cast<float4*>(states), reinterpret_cast<const float4*>(state_in), reinterpret_cast<float4*>(state_out), slopes, h,
-      nchunks, elems4, nblocks, bpc, n, p.reverse, skip_last, total);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  if (cudaGetLastError() != cudaSuccess) return LAB200_ERR_CUDA;
+  if ((rc = launch_kernel(la_scan_kernel, dim3(static_cast<unsigned>((total + 255) / 256)), 256, 0, st, true,
+                          reinterpret_cast<float4*>(states), reinterpret_cast<const float4*>(state_in), reinterpret_cast<float4*>(state_out),
+                          slopes, h, nchunks, elems4, nblocks, bpc, n, p.reverse, skip_last, total)) != LAB200_OK)
+    return rc;
   if (state_only || prefix_only) return LAB200_OK;
 
   p.chunk0 = 0;
@@ -340,9 +356,7 @@ int launch_dkdv_one(const CUtensorMap (&tm)[6], const LaDkdvParams& p, dim3 grid
     cudaGetLastError();
     return LAB200_ERR_CUDA;
   }
-  kern<<<grid, LD2_THREADS, smem, st>>>(tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], p);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
-  return cudaGetLastError() == cudaSuccess ? LAB200_OK : LAB200_ERR_CUDA;
+  return launch_kernel(kern, grid, LD2_THREADS, smem, st, !p.status.reset, tm[0], tm[1], tm[2], tm[3], tm[4], tm[5], p);
 }
 
 // lab200_la2_bwd computes dk and dv with the fused sweep (6 tensor passes instead of the 8 of two generic launches)

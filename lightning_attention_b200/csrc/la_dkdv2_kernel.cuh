@@ -120,6 +120,7 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const float s = p.slopes ? p.slopes[bh % p.h] : 0.f;
   const float s2 = -s * 1.4426950408889634f;
 
+  pdl_let_next_start();
   la_status_begin(p.status);
   if (tid == 0) {
     for (int i = 0; i < LD2_NUM_BARS; ++i) {
@@ -469,6 +470,7 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const bool st_row_valid = (r < p.d);
     const bool tracer = (w8 == 0 && lane == 0);
 
+    pdl_wait_for_previous();  // as in la_pipe_kernel.cuh
     float stt[SC];  // dKV[r][hf * SC ...]
 #pragma unroll
     for (int i = 0; i < SC; ++i) stt[i] = 0.f;

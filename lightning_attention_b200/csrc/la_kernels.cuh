@@ -133,6 +133,8 @@ __global__ void __launch_bounds__(256)
 la_scan_kernel(float4* __restrict__ states, const float4* __restrict__ init, float4* __restrict__ total,
                const float* __restrict__ slopes, int h, int nchunks, int elems4, int nblocks, int blocks_per_chunk, int n,
                int reverse, int skip_last, long long total4) {
+  pdl_let_next_start();
+  pdl_wait_for_previous();
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= total4) return;
   const int bh = static_cast<int>(idx / elems4);

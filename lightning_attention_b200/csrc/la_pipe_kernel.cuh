@@ -151,6 +151,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const float s = p.slopes ? p.slopes[bh % p.h] : 0.f;
   const float s2 = -s * 1.4426950408889634f;
 
+  pdl_let_next_start();
   la_status_begin(p.status);
   if (tid == 0) {
     for (int i = 0; i < LAP_NUM_BARS; ++i) {
@@ -435,6 +436,9 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const bool st_row_valid = WIDE ? (st_row < p.dk) : ((r < DV) && (dv_off + r < p.dv));
     const bool store_thread = (w8 == 0 && lane == 0);
 
+    // The tensors of the call are complete before its first kernel starts; the states are written by the kernels in front of this one.
+    // Output tiles and scaled copies follow this in program order.
+    if (MODE == 0 || have_state_in) pdl_wait_for_previous();
     float stt[SC];
 #pragma unroll
     for (int i = 0; i < SC; ++i) stt[i] = 0.f;
@@ -615,6 +619,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
       if (MODE == 0 && has_next && !scale_bm(it + 1)) { LAP_FAIL(LA_ERR_WAIT_MMA1) break; }
     }
+    if (MODE != 0) pdl_wait_for_previous();  // the kernel in front may still be reading the states of the product before
     if (*abort_flag == 0 && p.state_out != nullptr && st_row_valid) {
       float* dst = p.state_out + (static_cast<size_t>(bh) * p.state_slots + chunk) * p.dv * p.dk;
       if constexpr (WIDE) {

@@ -139,6 +139,12 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// Programmatic dependent launch: the kernels of one call overlap the start of each with the end of the one before. A kernel lets the
+// next one start as soon as all its own CTAs run, and waits for the one before (its completion, and with it that of all earlier
+// ones) in front of the first access to anything that kernels of the same call write.
+__device__ __forceinline__ void pdl_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Register split between warpgroups: every warp of the warpgroup executes it, N the registers per thread it goes on with. The block
 // is launched with LAUNCHED per thread; setmaxnreg.inc takes only counts above the current one and .dec only counts below it
 // (the other way round is an illegal instruction), so the form is chosen here and an equal count issues neither.

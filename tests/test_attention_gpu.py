@@ -592,6 +592,48 @@ def test_backward_from_kept_chunk_states(cuda_lib, d, n, chunks):
     assert cuda_lib.lab200_la2_bwd_kept(*args, *outs, kept.data_ptr(), nbytes, ws.data_ptr(), nbytes, *one) != 0
 
 
+@pytest.mark.parametrize("b,h,n,d,e", [(1, 4, 300, 64, 64), (1, 8, 2048, 128, 128), (2, 3, 1213, 128, 64), (1, 4, 1500, 192, 192), (4, 32, 256, 128, 128)])
+def test_overlapping_launches_of_one_call(cuda_lib, b, h, n, d, e):
+    """The kernels of a call start while the one before ends: back-to-back calls that share one workspace, on a second stream beside
+    other calls, and captured in a graph, give what separated calls give, bit for bit."""
+    q, k, v, do = (t.detach() for t in make_inputs(b, h, n, d, e, torch.bfloat16, 1.0))
+    s = (la._build_slope_tensor(h).reshape(-1) * 0.1).to(DEV)
+    nbytes = cuda_lib.lab200_la2_bwd_workspace_bytes(b, h, n, d, e, 0)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+    def buffers():
+        return [torch.zeros_like(t) for t in (v, q, k, v)]
+    def call(outs, w, sync=False):
+        st = torch.cuda.current_stream().cuda_stream
+        tail = (w.data_ptr(), nbytes, b, h, n, d, e, 0, _lib.BF16, st)
+        assert cuda_lib.lab200_la2_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), s.data_ptr(), outs[0].data_ptr(), *tail) == 0
+        if sync:
+            torch.cuda.synchronize()
+        assert cuda_lib.lab200_la2_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), s.data_ptr(), do.data_ptr(), outs[1].data_ptr(),
+                                       outs[2].data_ptr(), outs[3].data_ptr(), *tail) == 0
+    ref = buffers()
+    call(ref, ws, sync=True)
+    torch.cuda.synchronize()
+    runs = [buffers() for _ in range(4)]
+    for r in runs:
+        call(r, ws)
+    side, other, ws2 = torch.cuda.Stream(), buffers(), torch.empty_like(ws)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call(other, ws2)
+    call(runs[0], ws)
+    torch.cuda.synchronize()
+    graph, captured = torch.cuda.CUDAGraph(), buffers()
+    with torch.cuda.graph(graph):
+        call(captured, ws)
+    graph.replay()
+    graph.replay()
+    torch.cuda.synchronize()
+    for r in runs + [other, captured]:
+        for x, y in zip(r, ref):
+            assert torch.equal(x, y)
+    assert cuda_lib.lab200_last_status() == 0
+
+
 def test_decode_step_against_numpy_oracle(cuda_lib):
     torch.manual_seed(23)
     b, h, d, e = 3, 5, 48, 80
