@@ -4,8 +4,9 @@
 //
 //   warp 0      TMA producer   loads A, Bm, C tiles of block i+1, i+2 into two shared-memory stages
 //   warp 1      MMA issuer     X_i = A State_i, D_i = C^T (w Bm), PC_i = P_i C, S_{i+1} = A Bm^T, in this order (one thread)
+//   warps 2-3   scaling        half of: Bm_i rows *= w_state (for D_i)
 //   warps 4-7   mask group     S_i (TMEM) -> decay mask -> P_i (bf16, back into TMEM over S)
-//   warps 8-15  state/output   Bm_i rows *= w_state (for D_i); D_i -> StateT = lambda^128 StateT + D_i (fp32 registers)
+//   warps 8-15  state/output   the other half; D_i -> StateT = lambda^128 StateT + D_i (fp32 registers)
 //                              -> bf16 copy for X_{i+1}; O_i = PC_i + w_out X_i -> swizzled shared-memory tile -> TMA store
 //
 // P never touches shared memory: it is written to TMEM with tcgen05.st and consumed by tcgen05.mma as the
@@ -25,7 +26,7 @@
 
 namespace lab200 {
 
-// Four warpgroups: loads and MMAs (two of its warps idle), mask, and two of the state/output group. The launch gives every thread
+// Four warpgroups: loads, MMAs and half of the Bm scaling, mask, and two of the state/output group. The launch gives every thread
 // 128 registers; the fp32 state and the tiles beside it need more, the issuing threads far less, so the warpgroups split what
 // the launch was given. At 128 for all, the loops spilled 124-144 bytes per thread, and what spills goes through the shared-memory
 // pipe that bounds the kernel: b4 h32 n2048 d=e=128 forward 53.4 -> 51.4 us, n32768 forward 851 -> 823.
@@ -33,6 +34,7 @@ constexpr int LAP_THREADS = 512;
 constexpr int LAP_REGS[3] = {56, 120, 168};
 static_assert(LAP_REGS[0] + LAP_REGS[1] + 2 * LAP_REGS[2] <= 512, "the split must not ask for more than the launch gave");
 constexpr int LAP_MASK_THREADS = 128, LAP_STATE_THREADS = 256;
+constexpr int LAP_SCALE_THREADS = 64;  // warps 2 and 3
 
 
 // barrier slots (each has one instance per stage, indexed by block modulo the stage count)
@@ -87,6 +89,30 @@ __device__ __forceinline__ bool lap_wait(uint32_t bar, uint32_t parity, volatile
   return true;
 }
 
+// NP 16-byte chunks of one 128-byte tile row times the row's factor, in place: positions rot, rot + 1, ... modulo 8. rot grows with the
+// row, so that the same step of eight neighbouring rows covers all banks. EXACT: by w in fp32, one rounding per element; else packed, by
+// w rounded to the 16-bit type.
+template <int FMT, bool EXACT, int NP>
+__device__ __forceinline__ void lap_scale(uint32_t row, int rot, float w) {
+  uint32_t u[NP][4];
+  const uint32_t w2 = pack2<FMT>(w, w);
+#pragma unroll
+  for (int c = 0; c < NP; ++c) ld_shared_v4(row + (((rot + c) & 7) << 4), u[c][0], u[c][1], u[c][2], u[c][3]);
+#pragma unroll
+  for (int c = 0; c < NP; ++c) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if constexpr (EXACT) {
+        const float2 f = unpack2<FMT>(u[c][j]);
+        u[c][j] = pack2<FMT>(f.x * w, f.y * w);
+      } else {
+        u[c][j] = mul2<FMT>(u[c][j], w2);
+      }
+    }
+    st_shared_v4(row + (((rot + c) & 7) << 4), u[c][0], u[c][1], u[c][2], u[c][3]);
+  }
+}
+
 template <int NKS, int NVS, int MODE, int FMT>
 __global__ void __launch_bounds__(LAP_THREADS, 1)
 la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -101,6 +127,9 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   constexpr int NAS = WIDE ? 0 : (NKS > NVS ? NKS : NVS);  // slabs from one A stage to the next (0: there is one)
   constexpr int NBS = lap_b_stages(NKS, MODE) > 1 ? NKS : 0;
   constexpr int NST = lap_stages(MODE, NKS);
+  // Warps 2 and 3 take half of the Bm scaling in the narrow block loop. In the state-only pass the state group has the time, and the
+  // wide widths (fp32 multiply, 48-64 KB) are slower with it: 4 x 16 x 4096 x 256 forward 244 -> 268 us.
+  constexpr bool HELP = MODE == 0 && !WIDE;
   constexpr int NCS = lap_c_slabs(NKS);
   constexpr uint32_t T_S = 0, T_OI = 128, T_OX = 128 + DV, T_D = 128 + 2 * DV;
   static_assert(T_D + (WIDE ? 2 * DV : DKP) <= 512, "TMEM budget");
@@ -156,7 +185,8 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   if (tid == 0) {
     for (int i = 0; i < LAP_NUM_BARS; ++i) {
       const uint32_t count = (i == LAP_P_READY) ? LAP_MASK_THREADS
-                           : (i == LAP_O_FREE || i == LAP_D_FREE || i == LAP_STATE_READY || i == LAP_O_STAGED || i == LAP_BM_SCALED) ? LAP_STATE_THREADS : 1u;
+                           : (i == LAP_O_FREE || i == LAP_D_FREE || i == LAP_STATE_READY || i == LAP_O_STAGED) ? LAP_STATE_THREADS
+                           : (i == LAP_BM_SCALED) ? LAP_STATE_THREADS + (HELP ? LAP_SCALE_THREADS : 0) : 1u;
       for (int j = 0; j < NST; ++j) mbar_init(bar(i, j), count);
     }
     *abort_flag = 0;
@@ -333,6 +363,37 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
       }
+    } else if (HELP) {
+      // ============================================ scaling ===============================================
+      // The state group is the busiest role: state update, output tile, then the scaling that the next D waits for (clock stamps of
+      // b4 h32 n2048 d=e=128: 3,600 of a block's 4,750 cycles; 4,350 with this). These two warps take half of every row of Bm (positions
+      // rot + 4 .. rot + 7 of each slab) as soon as S is done with it, two rows per thread. Forward 51.4 -> 49.7 us.
+      const int r0 = (warp - 2) * 32 + lane;
+      const int tail = p.n - (p.nblocks - 1) * LA_BLOCK;
+      const bool tail_fix = !reverse && tail < LA_BLOCK && blk_end == p.nblocks;  // see the state group
+      const float wa = ex2f(s2 * static_cast<float>(reverse ? r0 : LA_BLOCK - r0));
+      const float wb = ex2f(s2 * static_cast<float>(reverse ? r0 + 64 : LA_BLOCK - 64 - r0));
+      for (int j = 0; j < nb; ++j) {
+        const int st = stage_of(j);
+        bool ok = lap_wait(bar(LAP_S_READY, st), parity_of(j), abort_flag, budget);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) { LAP_FAIL(LA_ERR_WAIT_MMA1) break; }
+        if (s != 0.f) {
+          float w0 = wa, w1 = wb;
+          if (tail_fix && j == nb - 1) {
+            w0 = r0 < tail ? ex2f(s2 * static_cast<float>(tail - r0)) : 0.f;
+            w1 = r0 + 64 < tail ? ex2f(s2 * static_cast<float>(tail - r0 - 64)) : 0.f;
+          }
+          const uint32_t row = sB + st * NBS * SLAB + r0 * 128;
+#pragma unroll 1
+          for (int ks = 0; ks < NKS; ++ks) {
+            lap_scale<FMT, false, 4>(row + ks * SLAB, r0 + 4, w0);
+            lap_scale<FMT, false, 4>(row + ks * SLAB + 64 * 128, r0 + 4, w1);
+          }
+          fence_proxy_async_smem();
+        }
+        mbar_arrive(bar(LAP_BM_SCALED, st));
+      }
     }
   } else if (warp < 8) {
     regs_set<128, LAP_REGS[1]>();
@@ -422,13 +483,11 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const float w_out = reverse ? ex2f(s2 * static_cast<float>(LA_BLOCK - r)) : ex2f(s2 * static_cast<float>(r));
     const float decay_blk = ex2f(s2 * static_cast<float>(LA_BLOCK));
     const float w_state = reverse ? ex2f(s2 * static_cast<float>(r)) : ex2f(s2 * static_cast<float>(LA_BLOCK - r));
-    const uint32_t w_state2 = pack2<FMT>(w_state, w_state);
     // A forward-time sweep that ends in a ragged block (n not a multiple of 128): the state leaving that block is decayed
     // to token n, not to the end of the 128-token tile, so that state_out chains exactly (rows >= tail are zero padding).
     const int tail = p.n - (p.nblocks - 1) * LA_BLOCK;
     const bool tail_fix = !reverse && tail < LA_BLOCK && blk_end == p.nblocks;
     const float w_tail = (tail_fix && r < tail) ? ex2f(s2 * static_cast<float>(tail - r)) : 0.f;
-    const uint32_t w_tail2 = pack2<FMT>(w_tail, w_tail);
     const float decay_tail = ex2f(s2 * static_cast<float>(tail));
     // this thread's part of the state: row r (dv), columns hf SC + i (dk); wide: row hf 128 + r (dk), columns i (dv)
     const int st_row = WIDE ? hf * 128 + r : r;
@@ -481,53 +540,21 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       mbar_arrive(bar(LAP_STATE_READY, 0));  // state entering block 0
     }
 
-    // Bm rows of block j *= w_state(r), in place, for D_j: this thread's half of the row's 16-byte chunks.
+    // Bm rows of block j *= w_state(r), in place, for D_j: this thread's share of the row, or of the half that warps 2 and 3 leave.
     auto scale_bm = [&](int j) -> bool {
       const int st = stage_of(j);
       // S_j must be done with the unscaled tile (state-only mode: the tile must have landed)
       bool ok = lap_wait(bar(MODE == 0 ? LAP_S_READY : LAP_FULL_AB, st), parity_of(j), abort_flag, budget);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) return false;
-      if (WIDE && s != 0.f) {
-        // w in fp32 here: one rounding per element; two slabs at a time keep the registers in bounds
+      if (s != 0.f) {
         const float w = (tail_fix && j == nb - 1) ? w_tail : w_state;
         const uint32_t row = sB + st * NBS * SLAB + r * 128;
+        if constexpr (NKS == 2) {
+          lap_scale<FMT, false, HELP ? 4 : 8>(row + hf * SLAB, r, w);
+        } else {
 #pragma unroll 1
-        for (int ks = 0; ks < NKS; ++ks) {
-          uint32_t u[4][4];
-#pragma unroll
-          for (int c = 0; c < 4; ++c)  // positions rotate with the row: eight rows cover all banks
-            ld_shared_v4(row + ks * SLAB + (((hf * 4 + c + r) & 7) << 4), u[c][0], u[c][1], u[c][2], u[c][3]);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-#pragma unroll
-            for (int j2 = 0; j2 < 4; ++j2) {
-              const float2 f = unpack2<FMT>(u[c][j2]);
-              u[c][j2] = pack2<FMT>(f.x * w, f.y * w);
-            }
-            st_shared_v4(row + ks * SLAB + (((hf * 4 + c + r) & 7) << 4), u[c][0], u[c][1], u[c][2], u[c][3]);
-          }
-        }
-        fence_proxy_async_smem();
-      } else if (!WIDE && s != 0.f) {
-        const uint32_t w2 = (tail_fix && j == nb - 1) ? w_tail2 : w_state2;
-        constexpr int NCH = NKS * 4;  // chunks per thread
-        const uint32_t sBs = sB + st * NBS * SLAB;
-        uint32_t u[NCH][4];
-        uint32_t addr[NCH];
-#pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-          const int gch = hf * NCH + c;  // chunk index in the row, 0 .. NKS*8-1
-          const int ks = gch >> 3, p0 = gch & 7;
-          const int pos = (NCH >= 8) ? ((p0 + r) & 7) : ((p0 & 4) | ((p0 + r) & 3));  // spread the warp over the banks
-          addr[c] = sBs + ks * SLAB + r * 128 + (pos << 4);
-          ld_shared_v4(addr[c], u[c][0], u[c][1], u[c][2], u[c][3]);
-        }
-#pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-#pragma unroll
-          for (int j2 = 0; j2 < 4; ++j2) u[c][j2] = mul2<FMT>(u[c][j2], w2);
-          st_shared_v4(addr[c], u[c][0], u[c][1], u[c][2], u[c][3]);
+          for (int ks = 0; ks < NKS; ++ks) lap_scale<FMT, WIDE, HELP ? 2 : 4>(row + ks * SLAB, hf * (HELP ? 2 : 4) + r, w);
         }
         fence_proxy_async_smem();
       }
