@@ -21,7 +21,7 @@ namespace {
 
 constexpr size_t WS_HEADER = 256;            // status block in front of the workspace
 constexpr int SMEM_LIMIT = 232448;           // 227 KB opt-in dynamic shared memory per CTA
-constexpr long long WAIT_BUDGET = 2000000000LL;  // ~1 s of SM clocks per barrier wait
+constexpr long long WAIT_BUDGET = 2000000000LL;  // ~1 s of SM clocks per barrier wait, of which none passes while the kernel in front runs
 
 std::atomic<long long> g_launches{0};  // kernels launched by this library since load
 std::atomic<long long*> g_trace{nullptr};  // optional device buffer for per-block clock stamps

@@ -212,6 +212,7 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             LD2_WAIT(LD2_PV0_READY, 0, LA_ERR_WAIT_MMA1)
             load_v(1);
           }
+          pdl_wait_for_previous();  // the waits from here on follow from the state group's, see behind_previous in la_pipe_kernel.cuh
           for (int it = 0; it < nb; ++it) {
             if (it + 1 < nb) {
               // q and k of the next block go to L2 now, a block before their loads: those loads sit in the chains that bound
@@ -243,6 +244,7 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // =========================================== TMA stores =============================================
       // The two staged output tiles of a block leave in turn through the one staging buffer.
       if (issuer_lane(lane)) {
+        pdl_wait_for_previous();
         for (int it = 0; it < nb; ++it) {
           bool ok = true;
 #pragma unroll 1
@@ -308,6 +310,7 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           umma_commit(bar(LD2_QP_DONE, it));
           LD2_TRACE(1, it)
           LD2_EV(1)
+          if (it == 0) pdl_wait_for_previous();
           if (have_state) {
             LD2_WAIT(LD2_STATE_READY, it, LA_ERR_WAIT_MMA2)
             tc_fence_after_sync();
@@ -454,6 +457,7 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (!alive) LD2_FAIL(LA_ERR_WAIT_MMA1)
     for (int it = 0; it < nb && alive; ++it) {
       alive = pass(1, it);
+      if (it == 0) pdl_wait_for_previous();
       if (alive && it + 1 < nb) alive = pass(0, it + 1);
       if (!alive) LD2_FAIL(LA_ERR_WAIT_MMA1)
     }

@@ -176,6 +176,11 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const int nk16 = p.dk >> 4;
   const long long budget = p.wait_budget;
   const bool have_state_in = (p.state_in != nullptr);
+  // The state group waits for the kernel in front before it touches chunk states or outputs. A bounded wait on anything that follows
+  // from there must not start earlier: its budget is for this CTA's own work, and the kernel in front may run for any time (one
+  // narrow pair of 60 million tokens in one chunk: longer than the budget). So every role passes the same point before its first
+  // such wait; what needs only loads and S of block 0 stays in front of it.
+  const bool behind_previous = MODE == 0 || have_state_in;
 
   const float s = p.slopes ? p.slopes[bh % p.h] : 0.f;
   const float s2 = -s * 1.4426950408889634f;
@@ -242,6 +247,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int ks = 0; ks < NKS; ++ks)
               tma_load_3d(sB + (st * NBS + ks) * SLAB, &tmB, ks * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_AB, st));
           };
+          if (behind_previous && it == (NAS == 0 ? 1 : NST)) pdl_wait_for_previous();
           if (NBS != 0 && it >= NST) {
             if (!lap_wait(bar(MODE == 0 ? LAP_PC_DONE : LAP_D_DONE, st), prev_par, abort_flag, budget)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
           }
@@ -271,6 +277,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             tma_load_3d(sC + (st * NCS + vs) * SLAB, &tmC, dv_off + vs * 64, blk * LA_BLOCK, zc, bar(LAP_FULL_C, st));
         }
         if (MODE == 0 && alive && *abort_flag == 0) {
+          pdl_wait_for_previous();  // fewer blocks than stages: not passed yet
           for (int i = max(nb - 2, 0); i < nb; ++i) {
             if (!store_tile(i)) { LAP_FAIL(LA_ERR_WAIT_MMA2) break; }
           }
@@ -302,6 +309,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           alive = issue_S(0);
           if (!alive) LAP_FAIL(LA_ERR_WAIT_INPUT)
         }
+        if (behind_previous) pdl_wait_for_previous();
         for (int it = 0; it < nb && alive; ++it) {
           const int st = stage_of(it);
           const uint32_t par = parity_of(it);
@@ -393,6 +401,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           fence_proxy_async_smem();
         }
         mbar_arrive(bar(LAP_BM_SCALED, st));
+        if (j == 0) pdl_wait_for_previous();
       }
     }
   } else if (warp < 8) {
@@ -471,6 +480,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         tc_fence_before_sync();
         mbar_arrive(bar(LAP_P_READY, st));
         if (tracer) { LAP_TRACE(5, it) }
+        if (it == 0) pdl_wait_for_previous();
       }
     }
   } else {
@@ -497,7 +507,7 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     // The tensors of the call are complete before its first kernel starts; the states are written by the kernels in front of this one.
     // Output tiles and scaled copies follow this in program order.
-    if (MODE == 0 || have_state_in) pdl_wait_for_previous();
+    if (behind_previous) pdl_wait_for_previous();
     float stt[SC];
 #pragma unroll
     for (int i = 0; i < SC; ++i) stt[i] = 0.f;

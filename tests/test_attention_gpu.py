@@ -634,6 +634,44 @@ def test_overlapping_launches_of_one_call(cuda_lib, b, h, n, d, e):
     assert cuda_lib.lab200_last_status() == 0
 
 
+def test_bounded_waits_do_not_count_the_kernel_in_front(cuda_lib):
+    """One pair, one chunk: dq and dk+dv are one CTA each, so dk+dv starts on another SM as soon as dq runs and waits for all of it -
+    here for longer than the budget of a bounded wait (2e9 clocks), which has to begin behind that. Against the same gradients in
+    chunks (sums of the same bf16 products in another order, rounded copies may differ by one bf16 step)."""
+    d, stream = 16, torch.cuda.current_stream().cuda_stream
+    s = torch.tensor([0.02], device=DEV)
+
+    def bwd(x, n, chunks):
+        outs = [torch.empty_like(x) for _ in range(3)]
+        nbytes = cuda_lib.lab200_la2_bwd_workspace_bytes(1, 1, n, d, d, chunks)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+        p = x.data_ptr()
+        rc = cuda_lib.lab200_la2_bwd(p, p, p, s.data_ptr(), p, *(o.data_ptr() for o in outs), ws.data_ptr(), nbytes, 1, 1, n, d, d, chunks, _lib.BF16, stream)
+        assert rc == 0 and cuda_lib.lab200_read_status(ws.data_ptr(), stream) == 0
+        return outs
+
+    # the length at which dq takes 1.3 s, from a short one
+    m = 1 << 20
+    x = (0.3 * torch.randn((m, d), device=DEV)).bfloat16()
+    o, ws = torch.empty_like(x), torch.empty(256, dtype=torch.uint8, device=DEV)
+    t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    for ev in (None, t0, t1):
+        if ev is not None:
+            ev.record()
+        if ev is not t1:
+            assert cuda_lib.lab200_la_generic(x.data_ptr(), x.data_ptr(), x.data_ptr(), s.data_ptr(), o.data_ptr(), None, None, ws.data_ptr(), 256,
+                                              1, 1, m, d, d, 0, 0, 1, _lib.BF16, stream) == 0
+    torch.cuda.synchronize()
+    n = min(1 << 27, int(m * 1300.0 / t0.elapsed_time(t1)) // 128 * 128)
+    assert n >= 1 << 24
+    x = (0.3 * torch.randn((n, d), device=DEV)).bfloat16()
+    got, ref = bwd(x, n, 1), bwd(x, n, 0)
+    for g, r in zip(got, ref):
+        for a, b in zip(g.split(1 << 24), r.split(1 << 24)):
+            assert torch.linalg.vector_norm((a - b).float()) <= 2.0 ** -8 * torch.linalg.vector_norm(b.float())
+    assert cuda_lib.lab200_last_status() == 0
+
+
 def test_decode_step_against_numpy_oracle(cuda_lib):
     torch.manual_seed(23)
     b, h, d, e = 3, 5, 48, 80
