@@ -135,9 +135,17 @@ struct Sizes {
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 const float* float_ptr(const Tensor& s) { return s.defined() ? static_cast<const float*>(s.const_data_ptr()) : nullptr; }
 
+// `t` in the layout of the call, copied if it has another one: a gradient, or a saved tensor. What saved-tensor hooks return has the
+// values of what was packed but often other strides (a copy through pinned host memory comes back contiguous).
+Tensor in_layout(const Tensor& t, bool bnhd) {
+  if (!bnhd) return t.contiguous();
+  return is_bnhd(t) ? t : empty_like_layout(t.size(0), t.size(1), t.size(2), t.size(3), t, true).copy_(t);
+}
+
 // ---- attention -------------------------------------------------------------------------------------------------------------
-// Same protocol as LightningAttention2 / LightningAttention2NoDecay in lightning_attn2.py: where the library cuts the sequence into
-// chunks and d == e, the forward pass keeps its workspace, and the first backward pass reads its chunk states transposed.
+// Where the library cuts the sequence into chunks and d == e, the forward pass saves its workspace too, and backward passes read its
+// chunk states transposed (they leave them as they are). It is saved like the other tensors, so that saved-tensor hooks have it as
+// well: checkpointing then keeps none from the forward pass, and takes the one of the recomputed pass.
 struct Attention : torch::autograd::Function<Attention> {
   static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<Tensor>& s_opt, bool bnhd) {
     const Tensor s = s_opt.has_value() ? *s_opt : Tensor();
@@ -149,27 +157,30 @@ struct Attention : torch::autograd::Function<Attention> {
     Tensor ws = workspace(bytes, q);
     check(g_api.la2_fwd(q.const_data_ptr(), k.const_data_ptr(), v.const_data_ptr(), float_ptr(s), o.mutable_data_ptr(), ws.mutable_data_ptr(),
                         bytes, z.b, z.h, z.n, z.d, z.e, 0, z.dt, stream_of(q)), "lab200_la2_fwd");
-    if (z.d == z.e && g_api.plan_chunks(z.b * z.h, z.n, z.d, z.e) > 1) ctx->saved_data["kept"] = ws;
+    const bool keep = z.d == z.e && g_api.plan_chunks(z.b * z.h, z.n, z.d, z.e) > 1;
     ctx->saved_data["bnhd"] = bnhd;
-    ctx->save_for_backward({q, k, v, s});
+    ctx->save_for_backward({q, k, v, s, keep ? ws : Tensor()});
     return o;
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list saved = ctx->get_saved_variables();
-    const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &s = saved[3];
     const bool bnhd = ctx->saved_data["bnhd"].toBool();
-    Tensor kept;  // given back with the first backward pass; a second one computes its states again
-    const auto it = ctx->saved_data.find("kept");
-    if (it != ctx->saved_data.end()) {
-      kept = it->second.toTensor();
-      ctx->saved_data.erase(it);
-    }
-    const c10::cuda::CUDAGuard guard(q.device());
+    Tensor go = grads[0], s = saved[3], kept = saved[4];
+    const at::IntArrayRef lead = go.sizes().slice(0, 3);
+    for (int i = 0; i < 3; ++i)
+      TORCH_CHECK(saved[i].defined() && saved[i].dim() == 4 && saved[i].sizes().slice(0, 3) == lead && saved[i].scalar_type() == go.scalar_type() &&
+                  saved[i].device() == go.device(), "lightning attention backward: saved-tensor hooks returned another shape, dtype or device");
+    TORCH_CHECK(saved[1].sizes() == saved[0].sizes() && saved[2].sizes() == go.sizes() && (!s.defined() || s.numel() >= go.size(1)),
+                "lightning attention backward: saved-tensor hooks returned another shape, dtype or device");
+    const c10::cuda::CUDAGuard guard(go.device());
+    if (s.defined() && !plain_slopes(s, go)) s = s.to(go.device(), at::kFloat).contiguous();
+    const Tensor q = in_layout(saved[0], bnhd), k = in_layout(saved[1], bnhd), v = in_layout(saved[2], bnhd);
+    go = in_layout(go, bnhd);
     const Sizes z(q, v, bnhd);
-    Tensor go = grads[0];
-    if (!bnhd) go = go.contiguous();
-    else if (!is_bnhd(go)) go = empty_like_layout(z.b, z.h, z.n, z.e, go, true).copy_(go);
+    if (kept.defined() && !(kept.scalar_type() == at::kByte && kept.device() == q.device() && kept.is_contiguous() && aligned16(kept) &&
+                            static_cast<size_t>(kept.numel()) == g_api.workspace_bytes(z.b * z.h, z.n, z.d, z.e, 0)))
+      kept = Tensor();  // not what was saved: the states are computed again
     raise_on_device_status(q);
     Tensor dq = empty_like_layout(z.b, z.h, z.n, z.d, q, bnhd), dk = empty_like_layout(z.b, z.h, z.n, z.d, q, bnhd);
     Tensor dv = empty_like_layout(z.b, z.h, z.n, z.e, q, bnhd);
