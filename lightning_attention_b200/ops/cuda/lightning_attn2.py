@@ -3,8 +3,8 @@
 Mirrors the operator layer of the reference: ``LightningAttention2`` / ``lightning_attn2``
 (lightning_attn/ops/triton/lightning_attn2.py:398-507) and ``LightningAttention2NoDecay`` /
 ``lightning_attn2_no_decay`` (lightning_attn2_no_decay.py:367-471). Inputs are made contiguous,
-outputs are allocated here with torch, (q, k, v, s) are saved for backward, and ``s`` receives no
-gradient, exactly as there. All device work goes through the C ABI on the current CUDA stream.
+outputs are allocated here with torch, (q, k, v, s) are saved for backward (with the chunk states, where
+the backward pass can take them over), and ``s`` receives no gradient, as there. All device work goes through the C ABI on the current CUDA stream.
 
 The public operators at the end try the native call path first (csrc/host_ops.cpp: the same checks, allocations, protocol and
 C-ABI calls without Python in between), which answers None to every call that is not of the common form.
@@ -205,8 +205,8 @@ def la_dkdv(q, k, v, s, do, state_in=None, chunks=0, resume_from=None):
     return dk, dv
 
 
-def _fwd(q, k, v, sl, chunks=0, bnhd=False):
-    """q, k, v all in one layout: (b, h, n, dim) contiguous, or (bnhd=True) views of (b, n, h, dim) tensors."""
+def _fwd_ws(q, k, v, sl, chunks=0, bnhd=False):
+    """(o, workspace); q, k, v all in one layout: (b, h, n, dim) contiguous, or (bnhd=True) views of (b, n, h, dim) tensors."""
     b, h, n, d = q.shape
     e = v.shape[-1]
     o = _empty_out(b, h, n, e, q.dtype, q.device, bnhd)
@@ -219,10 +219,15 @@ def _fwd(q, k, v, sl, chunks=0, bnhd=False):
                               nbytes, b, h, n, d, e, int(chunks), _lib.dtype_code(q.dtype) | (LAYOUT_BNHD if bnhd else 0),
                               _lib.stream_ptr(q.device))
     _lib.check(rc, "lab200_la2_fwd")
-    return o
+    return o, ws
 
 
-def _bwd(q, k, v, sl, do, chunks=0, bnhd=False):
+def _fwd(q, k, v, sl, chunks=0, bnhd=False):
+    return _fwd_ws(q, k, v, sl, chunks, bnhd)[0]
+
+
+def _bwd(q, k, v, sl, do, chunks=0, bnhd=False, kept=None):
+    """kept: the forward's workspace, if it holds chunk states that dq can read transposed (`_chunked`)."""
     b, h, n, d = q.shape
     e = v.shape[-1]
     dq = _empty_out(b, h, n, d, q.dtype, q.device, bnhd)
@@ -230,12 +235,18 @@ def _bwd(q, k, v, sl, do, chunks=0, bnhd=False):
     dv = _empty_out(b, h, n, e, q.dtype, q.device, bnhd)
     _lib.raise_on_device_status(q.device)
     L = _lib.lib()
+    dt = _lib.dtype_code(q.dtype) | (LAYOUT_BNHD if bnhd else 0)
+    ptrs = [q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.ptr(sl), do.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()]
     with torch.cuda.device(q.device):  # the chunk plan depends on the SM count of the tensors' device
         nbytes = L.lab200_la2_bwd_workspace_bytes(b, h, n, d, e, chunks)
         ws = _workspace(nbytes, q.device)
-        rc = L.lab200_la2_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.ptr(sl), do.data_ptr(), dq.data_ptr(),
-                              dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), nbytes, b, h, n, d, e, int(chunks),
-                              _lib.dtype_code(q.dtype) | (LAYOUT_BNHD if bnhd else 0), _lib.stream_ptr(q.device))
+        if kept is not None and not (kept.dtype == torch.uint8 and kept.device == q.device and kept.is_contiguous() and kept.data_ptr() % 16 == 0
+                                     and kept.numel() == L.lab200_la_workspace_bytes(b * h, n, d, e, chunks)):
+            kept = None  # not what was saved: the states are computed again
+        if kept is not None:
+            rc = L.lab200_la2_bwd_kept(*ptrs, kept.data_ptr(), kept.numel(), ws.data_ptr(), nbytes, b, h, n, d, int(chunks), dt, _lib.stream_ptr(q.device))
+        else:
+            rc = L.lab200_la2_bwd(*ptrs, ws.data_ptr(), nbytes, b, h, n, d, e, int(chunks), dt, _lib.stream_ptr(q.device))
     _lib.check(rc, "lab200_la2_bwd")
     return dq, dk, dv
 
@@ -249,21 +260,14 @@ def _chunked(q, v):
         return d == e and _lib.lib().lab200_la_plan_chunks(b * h, n, d, e) > 1
 
 
-def _fwd_keep(q, k, v, s):
-    """Forward that keeps its chunk states (KV prefixes, (e, d) per chunk) for the backward pass."""
-    o, _, handle = la_generic(q, k, v, s, keep_workspace=True)
-    return o, handle
-
-
-def _bwd_from_kept(q, k, v, s, do, handle):
-    """Backward in chunk mode with d == e: dq takes the forward's chunk states transposed, dv takes dk's; only dk's
-    (reverse-time sums of q^T do) are computed here."""
-    dq, _ = la_generic(do, v, k, s, resume_from=handle, resume_swapped=True, rebase=False)
-    if dkdv_fused_supported(q.shape[-1], v.shape[-1]):
-        return (dq,) + la_dkdv(q, k, v, s, do)
-    dk, _, h2 = la_generic(v, do, q, s, reverse=True, keep_workspace=True)
-    dv, _ = la_generic(k, q, do, s, reverse=True, resume_from=h2, resume_swapped=True, rebase=False)
-    return dq, dk, dv
+def _saved_for_bwd(q, k, v, do, bnhd):
+    """q, k, v, do in the layout of the call. Saved-tensor hooks return the values of what was packed, often in other strides."""
+    for t in (q, k, v):
+        if t.dim() != 4 or t.shape[:3] != do.shape[:3] or t.dtype != do.dtype or t.device != do.device:
+            raise RuntimeError("lightning attention backward: saved-tensor hooks returned another shape, dtype or device")
+    if k.shape != q.shape or v.shape != do.shape:
+        raise RuntimeError("lightning attention backward: saved-tensor hooks returned another shape, dtype or device")
+    return [_to_layout(t, bnhd) for t in (q, k, v, do)]
 
 
 def _check_inputs(q, k, v):
@@ -288,26 +292,16 @@ class LightningAttention2(torch.autograd.Function):
         bnhd = _use_bnhd(q, k, v)  # read (b, n, h, dim) projections in place, write o the same way: no transposing copies
         q, k, v = (_to_layout(t, bnhd) for t in (q, k, v))
         s = s.contiguous()
-        sl = _slopes_arg(s, q.shape[1], q.device)
-        ctx.kept = None
         ctx.bnhd = bnhd
-        if _chunked(q, v):
-            o, ctx.kept = _fwd_keep(q, k, v, s)
-        else:
-            o = _fwd(q, k, v, sl, bnhd=bnhd)
-        ctx.save_for_backward(q, k, v, s)
+        o, ws = _fwd_ws(q, k, v, _slopes_arg(s, q.shape[1], q.device), bnhd=bnhd)
+        ctx.save_for_backward(q, k, v, s, ws if _chunked(q, v) else None)
         return o
 
     @staticmethod
     def backward(ctx, do):
-        q, k, v, s = ctx.saved_tensors
-        do = _to_layout(do, ctx.bnhd)
-        kept, ctx.kept = ctx.kept, None  # usable once: the transposed hand-over changes whose states they are
-        if kept is not None:
-            return _bwd_from_kept(q, k, v, s, do, kept) + (None,)
-        sl = _slopes_arg(s, q.shape[1], q.device)
-        dq, dk, dv = _bwd(q, k, v, sl, do, bnhd=ctx.bnhd)
-        return dq, dk, dv, None
+        q, k, v, s, kept = ctx.saved_tensors
+        q, k, v, do = _saved_for_bwd(q, k, v, do, ctx.bnhd)
+        return _bwd(q, k, v, _slopes_arg(s, q.shape[1], q.device), do, bnhd=ctx.bnhd, kept=kept) + (None,)
 
 
 class LightningAttention2NoDecay(torch.autograd.Function):
@@ -318,24 +312,16 @@ class LightningAttention2NoDecay(torch.autograd.Function):
         _check_inputs(q, k, v)
         bnhd = _use_bnhd(q, k, v)
         q, k, v = (_to_layout(t, bnhd) for t in (q, k, v))
-        ctx.kept = None
         ctx.bnhd = bnhd
-        if _chunked(q, v):
-            o, ctx.kept = _fwd_keep(q, k, v, None)
-        else:
-            o = _fwd(q, k, v, None, bnhd=bnhd)
-        ctx.save_for_backward(q, k, v)
+        o, ws = _fwd_ws(q, k, v, None, bnhd=bnhd)
+        ctx.save_for_backward(q, k, v, ws if _chunked(q, v) else None)
         return o
 
     @staticmethod
     def backward(ctx, do):
-        q, k, v = ctx.saved_tensors
-        do = _to_layout(do, ctx.bnhd)
-        kept, ctx.kept = ctx.kept, None
-        if kept is not None:
-            return _bwd_from_kept(q, k, v, None, do, kept)
-        dq, dk, dv = _bwd(q, k, v, None, do, bnhd=ctx.bnhd)
-        return dq, dk, dv
+        q, k, v, kept = ctx.saved_tensors
+        q, k, v, do = _saved_for_bwd(q, k, v, do, ctx.bnhd)
+        return _bwd(q, k, v, None, do, bnhd=ctx.bnhd, kept=kept)
 
 
 def lightning_attn_prefill(q, k, v, s=None, kv_state=None):

@@ -77,11 +77,15 @@ def _odd_strides(t):
 @pytest.mark.parametrize("b,h,n,d,e,bnhd", [(1, 4, 1000, 128, 128, True), (1, 4, 1000, 128, 128, False), (2, 3, 300, 64, 96, True),
                                             (4, 32, 130, 128, 128, True), (1, 2, 700, 192, 192, False)])
 @pytest.mark.parametrize("decay", [True, False])
-def test_saved_tensor_hooks_that_return_another_layout(cuda_lib, b, h, n, d, e, bnhd, decay):
+@pytest.mark.parametrize("cls", [False, True], ids=["native", "class"])
+def test_saved_tensor_hooks_that_return_another_layout(cuda_lib, b, h, n, d, e, bnhd, decay, cls):
     """Cut into chunks and not; what comes back has the values that were packed, in other strides: the gradients are the same."""
     ts, do = _tensors(b, h, n, d, e, bnhd)
     s = la._build_slope_tensor(h).to(DEV) if decay else None
-    op = (lambda q, k, v: la.lightning_attn2(q, k, v, s)) if decay else la.lightning_attn2_no_decay
+    if cls:
+        op = (lambda q, k, v: la.LightningAttention2.apply(q, k, v, s)) if decay else la.LightningAttention2NoDecay.apply
+    else:
+        op = (lambda q, k, v: la.lightning_attn2(q, k, v, s)) if decay else la.lightning_attn2_no_decay
     assert (_lib.host().attn(*ts, s) if decay else _lib.host().attn_no_decay(*ts)) is not None
     ref = _grads(op, ts, do)
     hooks = [torch.autograd.graph.saved_tensors_hooks(lambda t: t, f) for f in (lambda t: t.contiguous().clone(), _odd_strides)]
