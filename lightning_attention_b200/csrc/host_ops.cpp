@@ -263,6 +263,17 @@ Tensor row_grad(const Tensor& g, const Tensor& x) {
   return g.contiguous().to(x.scalar_type());
 }
 
+// Saved rows and their 1 / rms, from whatever strides saved-tensor hooks return.
+Tensor saved_rows(const Tensor& x, const Tensor& g) {
+  TORCH_CHECK(x.defined() && x.dim() >= 1 && x.numel() == g.numel() && x.device() == g.device(), "norm backward: saved-tensor hooks returned another shape or device");
+  return x.contiguous();
+}
+Tensor saved_rstd(const Tensor& r, const Tensor& x) {
+  TORCH_CHECK(r.defined() && r.scalar_type() == at::kFloat && r.numel() == x.numel() / x.size(-1) && r.device() == x.device(),
+              "norm backward: saved-tensor hooks returned another shape, dtype or device");
+  return r.contiguous();
+}
+
 struct Norm : torch::autograd::Function<Norm> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, double eps) {
     const c10::cuda::CUDAGuard guard(x.device());
@@ -275,8 +286,8 @@ struct Norm : torch::autograd::Function<Norm> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &rstd = saved[1];
-    const c10::cuda::CUDAGuard guard(x.device());
+    const c10::cuda::CUDAGuard guard(grads[0].device());
+    const Tensor x = saved_rows(saved[0], grads[0]), rstd = saved_rstd(saved[1], x);
     const int64_t N = x.size(-1), M = x.numel() / N;
     const Tensor dy = row_grad(grads[0], x);
     Tensor dx = at::empty(dy.sizes(), x.options().requires_grad(false));
@@ -298,8 +309,11 @@ struct NormGate : torch::autograd::Function<NormGate> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &gate = saved[1], &rstd = saved[2];
-    const c10::cuda::CUDAGuard guard(x.device());
+    const c10::cuda::CUDAGuard guard(grads[0].device());
+    Tensor x = saved_rows(saved[0], grads[0]), gate = saved_rows(saved[1], grads[0]), rstd = saved_rstd(saved[2], x);
+    TORCH_CHECK(gate.scalar_type() == x.scalar_type() && gate.sizes() == x.sizes(), "norm backward: saved-tensor hooks returned another shape or dtype");
+    if (!aligned16(x)) x = x.clone();
+    if (!aligned16(gate)) gate = gate.clone();
     const int64_t N = x.size(-1), M = x.numel() / N;
     Tensor dy = row_grad(grads[0], x);
     if (!aligned16(dy)) dy = dy.clone();

@@ -32,7 +32,7 @@ class _SrmsNorm(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        x, rstd = ctx.saved_tensors
+        x, rstd = (t.contiguous() for t in ctx.saved_tensors)  # saved-tensor hooks may return other strides
         M, N = x.shape
         dy_arg = dy.reshape(-1, N).contiguous()
         assert dy_arg.numel() == x.numel(), "gradient and input sizes differ"  # srmsnorm.py:155-157
@@ -72,7 +72,8 @@ class _SrmsNormGate(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        x, g, rstd = ctx.saved_tensors
+        x, g, rstd = (t.contiguous() for t in ctx.saved_tensors)
+        x, g = _aligned16(x), _aligned16(g)
         M, N = x.shape
         dy_arg = dy.reshape(-1, N).contiguous()
         if dy_arg.dtype != x.dtype:

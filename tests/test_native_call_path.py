@@ -151,6 +151,25 @@ def test_norms_equal_the_python_functions(cuda_lib, dtype, shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("cls", [False, True], ids=["native", "class"])
+def test_norms_under_saved_tensor_hooks_that_return_another_layout(cuda_lib, dtype, cls):
+    x, g, dy = (torch.randn((6, 5, 512), device=DEV, dtype=dtype) for _ in range(3))
+    x.requires_grad_(), g.requires_grad_()
+    norm = (lambda t: _SrmsNorm.apply(t, 1e-6)) if cls else la.SimpleRMSNorm(512)
+    gated = (lambda t, u: _SrmsNormGate.apply(t, u, 1e-6)) if cls else la.srmsnorm_sigmoid_gate
+    ref = _grads(norm, [x], dy)[1:], _grads(gated, [x, g], dy)[1:]
+    apart = lambda t: torch.stack([t, t], -1)[..., 0]  # every second element: no dimension is contiguous
+    off = lambda t: torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view(t.shape)  # contiguous, not 16-byte aligned
+    for unpack in (_odd_strides, apart, off):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            y, z = norm(x), gated(x, g)
+        # rows that lost their alignment are reduced by another kernel, in another order: one rounding of the 16-bit result may differ
+        for a, b in zip(torch.autograd.grad(y, [x], dy) + torch.autograd.grad(z, [x, g], dy), ref[0] + ref[1]):
+            assert torch.linalg.vector_norm((a - b).float()) <= (2.0 ** -8 if dtype == torch.bfloat16 else 1e-6) * torch.linalg.vector_norm(b.float())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("bnhd", [False, True])
 def test_inference_calls_equal_the_general_product(cuda_lib, bnhd):
     ts, _ = _tensors(2, 3, 333, 64, 64, bnhd)
