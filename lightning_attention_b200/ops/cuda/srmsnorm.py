@@ -89,9 +89,15 @@ class _SrmsNormGate(torch.autograd.Function):
         return dx.reshape(dy.shape), dg.reshape(dy.shape), None
 
 
+def _native(x):
+    """Whether a norm of x may take the native call path: its outputs are plain tensors, the classes above return what
+    torch.empty_like makes of x, that is its own type."""
+    return type(x) in (torch.Tensor, torch.nn.Parameter) and not torch.compiler.is_compiling()
+
+
 def _srms_norm(x, eps):
     """_SrmsNorm through the native call path (csrc/host_ops.cpp) where the call has the common form, else through the class."""
-    if not torch.compiler.is_compiling():
+    if _native(x):
         y = _lib.host().norm(x, eps)
         if y is not None:
             return y
@@ -114,7 +120,7 @@ def srmsnorm_sigmoid_gate(x, gate, eps=1e-6):
     """SimpleRMSNorm(x) * sigmoid(gate). One fused kernel forward and one backward for rows of up to 16384 16-bit (8192
     fp32) elements that are a multiple of the 128-bit vector width; other rows compose SimpleRMSNorm with torch ops."""
     if _gate_rows_supported(x):
-        if not torch.compiler.is_compiling():
+        if _native(x):
             y = _lib.host().norm_gate(x, gate, eps)
             if y is not None:
                 return y

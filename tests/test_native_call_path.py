@@ -169,6 +169,25 @@ def test_norms_under_saved_tensor_hooks_that_return_another_layout(cuda_lib, dty
             assert torch.linalg.vector_norm((a - b).float()) <= (2.0 ** -8 if dtype == torch.bfloat16 else 1e-6) * torch.linalg.vector_norm(b.float())
 
 
+class _Marked(torch.Tensor):
+    """A subclass without a dispatch key of its own."""
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim", [64, 33])
+def test_norms_keep_the_type_of_a_tensor_subclass(cuda_lib, dim):
+    x, g, dy = (torch.randn((4, dim), device=DEV) for _ in range(3))
+    calls = [lambda t: la.SimpleRMSNorm(dim)(t), lambda t: la.srmsnorm_sigmoid_gate(t, g.as_subclass(type(t)))]
+    for call in calls:
+        ref = call(x)
+        assert type(ref) is torch.Tensor and type(call(torch.nn.Parameter(x))) is torch.Tensor
+        t = x.as_subclass(_Marked).requires_grad_()
+        y = call(t)
+        assert type(y) is _Marked and torch.equal(y.as_subclass(torch.Tensor), ref)
+        p = x.clone().requires_grad_()
+        assert torch.equal(torch.autograd.grad(y, t, dy)[0].as_subclass(torch.Tensor), torch.autograd.grad(call(p), p, dy)[0])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("bnhd", [False, True])
 def test_inference_calls_equal_the_general_product(cuda_lib, bnhd):
