@@ -920,9 +920,9 @@ int lab200_read_status(const void* workspace, void* stream) {
 int lab200_last_status(void) {
   int* word = host_status_word(false);
   if (!word) return 0;
-  const int v = *const_cast<volatile int*>(word);
-  if (v != 0) *const_cast<volatile int*>(word) = 0;
-  return v;
+  if (*const_cast<volatile int*>(word) == 0) return 0;
+  // one exchange: a report that arrives meanwhile is either returned or left, and of two threads only one gets it
+  return __atomic_exchange_n(word, 0, __ATOMIC_ACQ_REL);
 }
 
 int lab200_static_status(void* stream) {

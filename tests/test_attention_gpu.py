@@ -870,3 +870,48 @@ def test_expired_device_wait_reaches_the_caller_one_call_late(cuda_lib):
     torch.cuda.synchronize()
     assert torch.isfinite(o.float()).all()
     assert cuda_lib.lab200_last_status() == 0
+
+
+def test_a_report_reaches_one_caller_once(cuda_lib, tmp_path):
+    """Every expired wait is handed to exactly one of several threads that ask all the time (native threads: Python's take turns)."""
+    import ctypes
+    import subprocess
+    import threading
+    import time
+
+    src, so = tmp_path / "ask.cpp", tmp_path / "ask.so"
+    src.write_text("""
+#include <atomic>
+#include <thread>
+#include <vector>
+static std::atomic<int> stop{0};
+extern "C" void end() { stop = 1; }
+extern "C" int ask(int (*status)(), int threads, int code) {  // how often any thread was told `code`, or -1 on another answer
+  std::atomic<int> told{0}, other{0};
+  std::vector<std::thread> t;
+  for (int i = 0; i < threads; ++i)
+    t.emplace_back([&] {
+      while (!stop.load())
+        if (int v = status()) (v == code ? told : other)++;
+    });
+  for (auto& x : t) x.join();
+  return other.load() ? -1 : told.load();
+}
+""")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-pthread", str(src), "-o", str(so)], check=True)
+    A = ctypes.CDLL(str(so))
+    ws = torch.zeros(256, dtype=torch.uint8, device=DEV)
+    stream = torch.cuda.current_stream().cuda_stream
+    torch.cuda.synchronize()
+    assert cuda_lib.lab200_last_status() == 0
+    rounds, told = 300, []
+    asker = threading.Thread(target=lambda: told.append(A.ask(ctypes.cast(cuda_lib.lab200_last_status, ctypes.c_void_p), 4, 101)))
+    asker.start()
+    for _ in range(rounds):
+        assert cuda_lib.lab200_debug_wait_expiry(ws.data_ptr(), 256, 1000, stream) == 0
+        torch.cuda.synchronize()
+        time.sleep(0.001)  # the report is read before the next one is written
+    A.end()
+    asker.join(60)
+    assert told == [rounds]
+    assert cuda_lib.lab200_last_status() == 0
