@@ -90,8 +90,9 @@ int launch_kernel(K kern, dim3 grid, unsigned threads, size_t smem, cudaStream_t
   cfg.attrs = attr;
   cfg.numAttrs = follows ? 1 : 0;
   const cudaError_t rc = cudaLaunchKernelEx(&cfg, kern, args...);
+  const cudaError_t last = cudaGetLastError();  // read in any case: a refused launch must not be reported by the next call as well
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  return (rc == cudaSuccess && cudaGetLastError() == cudaSuccess) ? LAB200_OK : LAB200_ERR_CUDA;
+  return (rc == cudaSuccess && last == cudaSuccess) ? LAB200_OK : LAB200_ERR_CUDA;
 }
 
 struct Tiling {

@@ -915,3 +915,37 @@ extern "C" int ask(int (*status)(), int threads, int code) {  // how often any t
     asker.join(60)
     assert told == [rounds]
     assert cuda_lib.lab200_last_status() == 0
+
+
+def test_a_refused_launch_is_reported_by_its_own_call_only(cuda_lib):
+    """The runtime refuses launches into a capture that has been invalidated (here by waiting for the capturing stream): that call
+    returns an error, a decode step behind it is sound."""
+    import ctypes
+
+    R = ctypes.CDLL("libcudart.so.12")
+    b, h, n, d = 1, 2, 300, 64
+    q, k, v, _ = (t.detach() for t in make_inputs(b, h, n, d, d, torch.bfloat16, 1.0))
+    s = la._build_slope_tensor(h).reshape(-1).to(DEV)
+    o, state = la.lightning_attn_prefill(q, k, v, s)
+    tok = [t[:, :, 0].contiguous() for t in (q, k, v)]
+    want_state = state.clone()
+    want = la.lightning_attn_decode(*tok, s, want_state)
+    got = torch.empty_like(want)
+    nbytes = cuda_lib.lab200_la_workspace_bytes(b * h, n, d, d, 1)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+    torch.cuda.synchronize()
+    st, graph = ctypes.c_void_p(), ctypes.c_void_p()
+    assert R.cudaStreamCreateWithFlags(ctypes.byref(st), 1) == 0
+    assert R.cudaStreamBeginCapture(st, 1) == 0  # thread-local mode
+    assert R.cudaStreamSynchronize(st) != 0
+    R.cudaGetLastError()
+    refused = cuda_lib.lab200_la2_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), s.data_ptr(), o.data_ptr(), ws.data_ptr(), nbytes, b, h, n, d, d, 1,
+                                      _lib.BF16, st)
+    after = cuda_lib.lab200_la_decode_step(*(t.data_ptr() for t in tok), s.data_ptr(), state.data_ptr(), got.data_ptr(), b * h, h, d, d, _lib.BF16,
+                                           torch.cuda.current_stream().cuda_stream)
+    R.cudaStreamEndCapture(st, ctypes.byref(graph))
+    R.cudaGetLastError()
+    torch.cuda.synchronize()
+    assert R.cudaStreamDestroy(st) == 0
+    assert refused == 4 and after == 0
+    assert torch.equal(got, want) and torch.equal(state, want_state)
