@@ -1,6 +1,8 @@
 """ctypes binding of liblightning_b200.so. There is no fallback: a missing library is an error."""
 import ctypes
 import os
+import sysconfig
+import warnings
 
 import torch
 
@@ -85,16 +87,52 @@ _HOST_ENTRIES = ("lab200_error_string", "lab200_last_status", "lab200_la_plan_ch
                  "lab200_srmsnorm_gate_fwd", "lab200_srmsnorm_gate_bwd")
 
 
+HOST_PATH = os.path.join(_HERE, "_host_ops.so")
+
+
+def host_abi():
+    """What _host_ops.so has to be built for: it uses torch's C++ classes and the interpreter's, which have no stable binary form."""
+    return f"torch {torch.__version__} cxx11 {int(torch._C._GLIBCXX_USE_CXX11_ABI)} python {sysconfig.get_config_var('EXT_SUFFIX')}"
+
+
+def host_built_for(path=None):
+    """What the file was built for (its exported string), or None if there is none to be had."""
+    path = path or HOST_PATH
+    if not os.path.exists(path):
+        return None
+    try:
+        f = ctypes.CDLL(path).lab200_host_built_for
+    except (OSError, AttributeError):
+        return None
+    f.restype = ctypes.c_char_p
+    return f().decode()
+
+
+class _NoHost:
+    """Stands in for _host_ops where it cannot be had: every call is left to the Python operators."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def host():
-    """The native call path (_host_ops.so), bound to the entry points of the loaded library."""
+    """The native call path (_host_ops.so), bound to the entry points of the loaded library. The Python operators take every call as
+    well, so a file that is missing, does not load or was built for another torch costs time (one warning), not the call."""
     global _host
     if _host is None:
         L = lib()
-        try:
-            from . import _host_ops
-        except ImportError as ex:
-            raise ImportError(f"_host_ops.so is missing or does not load ({ex}): build it with "
-                              "`python -m lightning_attention_b200.build`") from ex
+        why = None
+        if host_built_for() != host_abi():
+            why = f"is missing, does not load or is built for {host_built_for()}, not for {host_abi()}"
+        else:
+            try:
+                from . import _host_ops
+            except ImportError as ex:
+                why = f"does not load ({ex})"
+        if why:
+            warnings.warn(f"{HOST_PATH} {why}: operators take the slower Python path; build it with `python -m lightning_attention_b200.build`")
+            _host = _NoHost()
+            return _host
         _host_ops.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in _HOST_ENTRIES})
         _host = _host_ops
     return _host

@@ -8,6 +8,8 @@ import shutil
 import subprocess
 import sys
 
+from . import _lib
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_NAME = "liblightning_b200.so"
 LIB_PATH = os.path.join(HERE, LIB_NAME)
@@ -22,7 +24,7 @@ NVCC_FLAGS = [
 ]
 
 
-HOST_PATH = os.path.join(HERE, "_host_ops.so")
+HOST_PATH = _lib.HOST_PATH
 HOST_SOURCES = [os.path.join(HERE, "csrc", "host_ops.cpp"), os.path.join(HERE, "..", "include", "lightning_b200.h")]
 
 
@@ -62,8 +64,8 @@ def build_host(verbose=False):
     cuda = os.path.dirname(os.path.dirname(find_nvcc()))
     inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
            os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
-    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DLAB200_HOST_ABI="{_lib.host_abi()}"']
     cmd += [a for d in inc for a in ("-isystem", d)] + ["-o", HOST_PATH, HOST_SOURCES[0], "-L" + os.path.join(root, "lib")]
     _run(cmd + ["-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python"], "g++", verbose)
     return HOST_PATH
@@ -73,7 +75,7 @@ def build(force=False, verbose=False):
     """Compile what is missing or older than its sources. Returns the path of the C-ABI library."""
     if force or not _newer(LIB_PATH, SOURCES + HEADERS):
         _run([find_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB_PATH] + SOURCES, "nvcc", verbose)
-    if force or not _newer(HOST_PATH, HOST_SOURCES):
+    if force or not _newer(HOST_PATH, HOST_SOURCES) or _lib.host_built_for(HOST_PATH) != _lib.host_abi():
         build_host(verbose)
     return LIB_PATH
 

@@ -337,6 +337,9 @@ std::optional<Tensor> norm_gate(const Tensor& x, const Tensor& gate, double eps)
 
 }  // namespace
 
+// What this file was compiled for, for a look before it is imported (_lib.py:host_abi).
+extern "C" __attribute__((visibility("default"))) const char* lab200_host_built_for() { return LAB200_HOST_ABI; }
+
 PYBIND11_MODULE(_host_ops, m) {
   m.def("bind", &bind);
   // The GIL is released, as ctypes does: a launch may have to wait for room in the stream's queue.

@@ -1,4 +1,7 @@
 """The operators' native call path (csrc/host_ops.cpp) against the Python autograd Functions it stands in for."""
+import subprocess
+import warnings
+
 import pytest
 import torch
 
@@ -17,6 +20,42 @@ def test_cpu_tensors_are_left_to_the_python_operators():
     for call in (lambda: la.lightning_attn2(x, x, x, torch.zeros(2)), lambda: la.SimpleRMSNorm(16)(x), lambda: la.srmsnorm_sigmoid_gate(x, x)):
         with pytest.raises(RuntimeError, match="CUDA tensors only"):
             call()
+
+
+@pytest.mark.parametrize("kind", ["missing", "garbage", "no string", "other torch"])
+def test_a_native_path_that_cannot_be_used_costs_one_warning(monkeypatch, tmp_path, kind):
+    path = tmp_path / "_host_ops.so"
+    if kind == "garbage":
+        path.write_bytes(b"not a library")
+    elif kind != "missing":
+        src = tmp_path / "x.c"
+        src.write_text("int x;" if kind == "no string" else 'const char* lab200_host_built_for(void) { return "torch 1.0"; }')
+        subprocess.run(["gcc", "-shared", "-fPIC", str(src), "-o", str(path)], check=True)
+    assert _lib.host_built_for() == _lib.host_abi()  # the file in the tree
+    monkeypatch.setattr(_lib, "HOST_PATH", str(path))
+    monkeypatch.setattr(_lib, "_host", None)
+    x = torch.zeros(1, 2, 16, 16, dtype=torch.bfloat16)
+    with pytest.warns(UserWarning, match="slower Python path"):
+        assert _lib.host().attn(x, x, x, torch.zeros(2)) is None
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        for call in (lambda: la.lightning_attn2(x, x, x, torch.zeros(2)), lambda: la.lightning_attn_decode(x, x, x, None, x), lambda: la.SimpleRMSNorm(16)(x)):
+            with pytest.raises(RuntimeError, match="CUDA tensors only"):
+                call()
+
+
+def test_the_build_sees_another_torch(monkeypatch):
+    """The native path is compiled anew when it was built for another torch, whatever the times of the files say."""
+    from lightning_attention_b200 import build
+
+    runs = []
+    monkeypatch.setattr(build, "build_host", lambda verbose=False: runs.append(1))
+    monkeypatch.setattr(build, "_newer", lambda *a: True)
+    build.build()
+    assert not runs
+    monkeypatch.setattr(_lib, "host_abi", lambda: "torch 99")
+    build.build()
+    assert runs == [1]
 
 
 def _tensors(b, h, n, d, e, bnhd, dtype=torch.bfloat16):
