@@ -594,29 +594,32 @@ def test_backward_from_kept_chunk_states(cuda_lib, d, n, chunks):
 
 @pytest.mark.parametrize("b,h,n,d,e", [(1, 4, 300, 64, 64), (1, 8, 2048, 128, 128), (2, 3, 1213, 128, 64), (1, 4, 1500, 192, 192), (4, 32, 256, 128, 128)])
 def test_overlapping_launches_of_one_call(cuda_lib, b, h, n, d, e):
-    """The kernels of a call start while the one before ends: back-to-back calls that share one workspace, on a second stream beside
-    other calls, and captured in a graph, give what separated calls give, bit for bit."""
-    q, k, v, do = (t.detach() for t in make_inputs(b, h, n, d, e, torch.bfloat16, 1.0))
+    """The kernels of a call start while the one before ends. One call on a poisoned workspace is compared with the fp32 recurrence;
+    back-to-back calls that share one workspace, on a second stream beside other calls, and captured in a graph, with workspace and
+    outputs poisoned (a state or tile read before it is written is then no other call's, but NaN), give the same, bit for bit."""
+    q, k, v, do = make_inputs(b, h, n, d, e, torch.bfloat16, 1.0)
     s = (la._build_slope_tensor(h).reshape(-1) * 0.1).to(DEV)
     nbytes = cuda_lib.lab200_la2_bwd_workspace_bytes(b, h, n, d, e, 0)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+    ws = torch.full((nbytes,), 255, dtype=torch.uint8, device=DEV)
     def buffers():
-        return [torch.zeros_like(t) for t in (v, q, k, v)]
-    def call(outs, w, sync=False):
+        return [torch.full_like(t, float("nan"), requires_grad=False) for t in (v, q, k, v)]
+    def call(outs, w):
         st = torch.cuda.current_stream().cuda_stream
         tail = (w.data_ptr(), nbytes, b, h, n, d, e, 0, _lib.BF16, st)
         assert cuda_lib.lab200_la2_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), s.data_ptr(), outs[0].data_ptr(), *tail) == 0
-        if sync:
-            torch.cuda.synchronize()
         assert cuda_lib.lab200_la2_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), s.data_ptr(), do.data_ptr(), outs[1].data_ptr(),
                                        outs[2].data_ptr(), outs[3].data_ptr(), *tail) == 0
     ref = buffers()
-    call(ref, ws, sync=True)
+    call(ref, ws)
     torch.cuda.synchronize()
-    runs = [buffers() for _ in range(4)]
-    for r in runs:
+    compare_with_torch_reference(q, k, v, do, s, ref, False, "overlapping launches")
+    runs = [buffers() for _ in range(6)]
+    for r in runs[:2]:
+        ws.fill_(255)
         call(r, ws)
-    side, other, ws2 = torch.cuda.Stream(), buffers(), torch.empty_like(ws)
+    for r in runs[2:]:
+        call(r, ws)
+    side, other, ws2 = torch.cuda.Stream(), buffers(), torch.full_like(ws, 255)
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
         call(other, ws2)
@@ -625,8 +628,11 @@ def test_overlapping_launches_of_one_call(cuda_lib, b, h, n, d, e):
     graph, captured = torch.cuda.CUDAGraph(), buffers()
     with torch.cuda.graph(graph):
         call(captured, ws)
-    graph.replay()
-    graph.replay()
+    for _ in range(2):
+        ws.fill_(255)
+        for t in captured:
+            t.fill_(float("nan"))
+        graph.replay()
     torch.cuda.synchronize()
     for r in runs + [other, captured]:
         for x, y in zip(r, ref):

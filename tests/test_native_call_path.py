@@ -107,6 +107,57 @@ def test_attention_equals_the_python_function(cuda_lib, b, h, n, d, e, bnhd, dec
         assert not fast(*ts).requires_grad
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,h,n,d", [(1, 4, 1000, 128), (4, 32, 130, 64)])
+def test_native_path_with_a_dispatch_mode_another_stream_and_two_threads(cuda_lib, b, h, n, d):
+    """A dispatch mode sees the Python functions' operations; a backward pass of a forward on a side stream runs there; two threads may
+    run the backward pass of one retained graph."""
+    import threading
+
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    ts, do = _tensors(b, h, n, d, d, False)
+    s = la._build_slope_tensor(h).to(DEV)
+    op = lambda q, k, v: la.lightning_attn2(q, k, v, s)
+    ref = _grads(op, ts, do)
+
+    class Seen(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            names.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    names = []
+    with Seen():
+        assert _lib.host().attn(*ts, s) is None
+        o = op(*ts)
+    assert any("empty" in x for x in names)
+    _same((o,) + torch.autograd.grad(o, ts, do), ref)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        # the copies are late on the side stream: a backward pass on another one would read them too early
+        torch.cuda._sleep(20_000_000)
+        late = [t.detach().clone().requires_grad_() for t in ts]
+        o = op(*late)
+    got = torch.autograd.grad(o, late, do)  # called with the default stream current
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    _same((o,) + got, ref)
+
+    o, res = op(*ts), [None, None]
+    def run(i):
+        res[i] = [torch.autograd.grad(o, ts, do, retain_graph=True) for _ in range(20)]
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for r in res:
+        for g in r:
+            _same(g, ref[1:])
+
+
 def _odd_strides(t):
     """The same values with the second dimension innermost (one-dimensional and byte tensors as they are)."""
     return t.transpose(1, -1).contiguous().transpose(1, -1) if t.dim() > 1 else t
