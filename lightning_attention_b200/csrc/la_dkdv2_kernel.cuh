@@ -212,7 +212,6 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             LD2_WAIT(LD2_PV0_READY, 0, LA_ERR_WAIT_MMA1)
             load_v(1);
           }
-          pdl_wait_for_previous();  // the waits from here on follow from the state group's, see behind_previous in la_pipe_kernel.cuh
           for (int it = 0; it < nb; ++it) {
             if (it + 1 < nb) {
               // q and k of the next block go to L2 now, a block before their loads: those loads sit in the chains that bound
@@ -221,6 +220,8 @@ la_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               for (int sl = 0; sl < 2; ++sl) tma_prefetch_l2_3d(&tmQ, sl * 64, blk_of(it + 1) * LA_BLOCK, zc);
               for (int sl = 0; sl < ND; ++sl) tma_prefetch_l2_3d(&tmK, sl * 64, blk_of(it + 1) * LA_BLOCK, zc);
             }
+            // the waits from here on follow from the state group's, see behind_previous in la_pipe_kernel.cuh
+            if (it == 0) pdl_wait_for_previous();
             if (it + 1 < nb) {
               LD2_WAIT(LD2_D_DONE, it, LA_ERR_WAIT_MMA2)
               load_q(it + 1);
