@@ -818,7 +818,7 @@ int lab200_la2_fwd_static(const void* q, const void* k, const void* v, const flo
     return LAB200_ERR_SCRATCH_LIMIT;
   void* scratch = nullptr;
   if ((rc = static_scratch_address(&scratch)) != LAB200_OK) return rc;
-  // the array keeps whatever the previous call left: the status word must start at zero; the chunk states
+  // the array keeps whatever the previous call left: the first kernel clears the status word; the chunk states
   // need no clearing because the state kernel writes every slot that the scan reads
   CallStatus status(scratch, nullptr);
   return la_generic_impl(q, k, v, slopes, o, nullptr, nullptr, scratch, LAB200_STATIC_SCRATCH_BYTES, b * h, h, n, d, e,

@@ -51,8 +51,8 @@ struct LaDkdvParams {
   int trace_blocks;
 };
 
-// Warpgroups and register split as in la_pipe_kernel.cuh; here the 128 registers of an even split spilled 36 bytes:
-// b2 h16 n4096 d=e=128 backward 130.5 -> 124.7 us, b4 h32 n32768 2045 -> 2000.
+// Warpgroups and register split as in la_pipe_kernel.cuh; here the 128 registers of an even split spilled 36 bytes,
+// this one 8 (24 at d, e <= 64), which is 8 local loads per block of a whole CTA at d=e=128: b2 h16 n4096 backward 130.5 -> 124.7 us.
 constexpr int LD2_THREADS = 512;
 constexpr int LD2_REGS[3] = {96, 128, 144};
 static_assert(LD2_REGS[0] + LD2_REGS[1] + 2 * LD2_REGS[2] <= 512, "the split must not ask for more than the launch gave");

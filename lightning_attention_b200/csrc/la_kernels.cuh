@@ -17,7 +17,7 @@
 //
 // The sequence is cut into blocks of 128 tokens. Per block (r, c = row indices inside the block):
 //     S      = A Bm^T                                   tcgen05.mma, fp32 in TMEM
-//     P      = S (.) M,  M[r,c] = lambda^|r-c| on the causal side, 0 elsewhere   (CUDA cores -> smem)
+//     P      = S (.) M,  M[r,c] = lambda^|r-c| on the causal side, 0 elsewhere   (CUDA cores, back into TMEM)
 //     O      = P C + diag(w_out) A State                two tcgen05.mma chains, combined in the epilogue
 //     StateT = lambda^128 StateT + C^T (diag(w_state) Bm)   tcgen05.mma + fp32 registers
 // with w_out(r) = lambda^r, w_state(r) = lambda^(128-r) in forward time and the two swapped in

@@ -29,7 +29,8 @@ namespace lab200 {
 // Four warpgroups: loads, MMAs and half of the Bm scaling, mask, and two of the state/output group. The launch gives every thread
 // 128 registers; the fp32 state and the tiles beside it need more, the issuing threads far less, so the warpgroups split what
 // the launch was given. At 128 for all, the loops spilled 124-144 bytes per thread, and what spills goes through the shared-memory
-// pipe that bounds the kernel: b4 h32 n2048 d=e=128 forward 53.4 -> 51.4 us, n32768 forward 851 -> 823.
+// pipe that bounds the kernel: b4 h32 n2048 d=e=128 forward 53.4 -> 51.4 us (at n32768 runs under the power cap differ by as much).
+// What still spills in the block loop: 60 bytes at dk > 192, 4 to 8 at dk <= 64 and on 64-wide slices of dk <= 128.
 constexpr int LAP_THREADS = 512;
 constexpr int LAP_REGS[3] = {56, 120, 168};
 static_assert(LAP_REGS[0] + LAP_REGS[1] + 2 * LAP_REGS[2] <= 512, "the split must not ask for more than the launch gave");
@@ -127,8 +128,9 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   constexpr int NAS = WIDE ? 0 : (NKS > NVS ? NKS : NVS);  // slabs from one A stage to the next (0: there is one)
   constexpr int NBS = lap_b_stages(NKS, MODE) > 1 ? NKS : 0;
   constexpr int NST = lap_stages(MODE, NKS);
-  // Warps 2 and 3 take half of the Bm scaling in the narrow block loop. In the state-only pass the state group has the time, and the
-  // wide widths (fp32 multiply, 48-64 KB) are slower with it: 4 x 16 x 4096 x 256 forward 244 -> 268 us.
+  // Warps 2 and 3 take half of the Bm scaling in the narrow block loop. In the state-only pass the state group has the time. The wide
+  // widths (fp32 multiply, 48-64 KB) were measured at dk = 256 only, where Bm has one stage, and are slower with it there (4 x 16 x
+  // 4096 x 256 forward 244 -> 268 us); 129 to 192, with two stages of Bm, follow that rule unmeasured.
   constexpr bool HELP = MODE == 0 && !WIDE;
   constexpr int NCS = lap_c_slabs(NKS);
   constexpr uint32_t T_S = 0, T_OI = 128, T_OX = 128 + DV, T_D = 128 + 2 * DV;
@@ -141,15 +143,15 @@ la_pipe_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
-  const uint32_t sA = base;                                         // 2 stages x NAS slabs, wide: 1 x NKS (MODE 0)
-  const uint32_t sB = sA + (MODE == 0 ? lap_a_slabs(NKS, NVS) * SLAB : 0);  // 2 stages x NKS slabs (NKS = 4, MODE 0: 1)
-  const uint32_t sC = sB + lap_b_stages(NKS, MODE) * NKS * SLAB;    // 2 stages x NCS slabs
+  const uint32_t sA = base;                                         // MODE 0 only: 2 stages x NAS slabs, wide: 1 x NKS
+  const uint32_t sB = sA + (MODE == 0 ? lap_a_slabs(NKS, NVS) * SLAB : 0);  // lap_b_stages x NKS slabs: 2 (NKS = 4: 1), state-only 3 (NKS = 4: 2)
+  const uint32_t sC = sB + lap_b_stages(NKS, MODE) * NKS * SLAB;    // NST stages x NCS slabs: 2, state-only 3 (NKS = 4: 2)
   // 16-bit state: NKS x [DV rows][128 B] (rows dv, columns dk); wide: [DKP rows][128 B] (rows dk, columns dv) (MODE 0). The second
   // M = 128 tile of D at NKS = 3 reads one slab behind its Bm stage: that is the other stage or C, and only reaches accumulator
   // rows that nobody reads.
   const uint32_t sS = sC + NST * NCS * SLAB;
   // Output tiles are staged in the C stage of their own block (free once P C is done) and leave by TMA store.
-  const uint32_t sBar = sS + (MODE == 0 ? NKS * DV * 128 : 0);      // 2 x LAP_NUM_BARS mbarriers
+  const uint32_t sBar = sS + (MODE == 0 ? NKS * DV * 128 : 0);      // NST x LAP_NUM_BARS mbarriers
   const uint32_t sMisc = sBar + NST * LAP_NUM_BARS * 8;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_raw + (sMisc - raw));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_raw + (sMisc + 4 - raw));

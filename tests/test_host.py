@@ -176,4 +176,4 @@ def test_backward_workspace_covers_every_product_of_the_backward_pass():
 
 def test_status_queries_need_no_gpu():
     L = _lib.lib()
-    assert L.lab200_last_status() == 0  # no device, no ring: nothing to report
+    assert L.lab200_last_status() == 0  # no device, no word: nothing to report
