@@ -8,7 +8,11 @@ import shutil
 import subprocess
 import sys
 
-from . import _lib
+if __package__:
+    from . import _lib
+else:  # run by its path
+    sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    from lightning_attention_b200 import _lib
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_NAME = "liblightning_b200.so"

@@ -1,5 +1,6 @@
 """The operators' native call path (csrc/host_ops.cpp) against the Python autograd Functions it stands in for."""
 import subprocess
+import sys
 import warnings
 
 import pytest
@@ -56,6 +57,13 @@ def test_the_build_sees_another_torch(monkeypatch):
     monkeypatch.setattr(_lib, "host_abi", lambda: "torch 99")
     build.build()
     assert runs == [1]
+
+
+def test_the_build_runs_by_its_path_as_well():
+    from lightning_attention_b200 import build
+
+    r = subprocess.run([sys.executable, build.__file__], capture_output=True, text=True)  # up to date: nothing is compiled
+    assert r.returncode == 0 and r.stdout.strip() == build.LIB_PATH, r.stderr
 
 
 def _tensors(b, h, n, d, e, bnhd, dtype=torch.bfloat16):
